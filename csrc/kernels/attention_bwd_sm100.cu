@@ -153,7 +153,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
   if (warp == 9) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_q);
       tma_prefetch_desc(&map_k);
       tma_prefetch_desc(&map_v);
@@ -189,7 +189,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
   } else if (warp == 8) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_dkv = make_idesc_bf16(128, D, 1, 1);
       constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, 0, 1);
@@ -211,8 +211,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         for (int c = 0; c < KCH; ++c)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_ss(tmem_base + TM_S, make_smem_desc_sw128(q_base + c * 16384 + k * 32, 16, 1024),
-                    make_smem_desc_sw128(k_base + c * 16384 + k * 32, 16, 1024), idesc_s, (c | k) ? 1u : 0u);
+            umma_ss(tmem_base + TM_S, desc_at(make_smem_desc_sw128(q_base, 16, 1024), c * 16384 + k * 32),
+                    desc_at(make_smem_desc_sw128(k_base, 16, 1024), c * 16384 + k * 32), idesc_s, (c | k) ? 1u : 0u);
         umma_commit(s_full);
         if (PIPELINED && t > 0) mbar_wait(dp_free, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
         mbar_wait(&do_full[s], ph, abort_flag, p.status, TB_ERR_WAIT_FULL);
@@ -221,8 +221,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         for (int c = 0; c < KCH; ++c)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_ss(tmem_base + TM_DP, make_smem_desc_sw128(do_base + c * 16384 + k * 32, 16, 1024),
-                    make_smem_desc_sw128(v_base + c * 16384 + k * 32, 16, 1024), idesc_s, (c | k) ? 1u : 0u);
+            umma_ss(tmem_base + TM_DP, desc_at(make_smem_desc_sw128(do_base, 16, 1024), c * 16384 + k * 32),
+                    desc_at(make_smem_desc_sw128(v_base, 16, 1024), c * 16384 + k * 32), idesc_s, (c | k) ? 1u : 0u);
         umma_commit(dp_full);
       };
       if (PIPELINED && n_it > 0) issue_scores(0);
@@ -242,18 +242,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ss(tmem_base + TM_DV, make_smem_desc_sw128(p_base + kk * 2048, 16384, 1024),
-                  make_smem_desc_sw128(do_base + kk * 2048, 16384, 1024), idesc_dkv, (t | kk) ? 1u : 0u);
+          umma_ss(tmem_base + TM_DV, desc_at(make_smem_desc_sw128(p_base, 16384, 1024), kk * 2048),
+                  desc_at(make_smem_desc_sw128(do_base, 16384, 1024), kk * 2048), idesc_dkv, (t | kk) ? 1u : 0u);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ss(tmem_base + TM_DK, make_smem_desc_sw128(ds_base + kk * 2048, 16384, 1024),
-                  make_smem_desc_sw128(q_base + kk * 2048, 16384, 1024), idesc_dkv, (t | kk) ? 1u : 0u);
+          umma_ss(tmem_base + TM_DK, desc_at(make_smem_desc_sw128(ds_base, 16384, 1024), kk * 2048),
+                  desc_at(make_smem_desc_sw128(q_base, 16384, 1024), kk * 2048), idesc_dkv, (t | kk) ? 1u : 0u);
         if (D == 64 && t > 0) mbar_wait(dq_empty, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_ss(tmem_base + TM_DQ,
-                  make_smem_desc_sw128(ds_base + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                  make_smem_desc_sw128(k_base + kk * 2048, 16384, 1024), idesc_dq, kk ? 1u : 0u);
+                  desc_at(make_smem_desc_sw128(ds_base, 16, 1024), (kk >> 2) * 16384 + (kk & 3) * 32),
+                  desc_at(make_smem_desc_sw128(k_base, 16384, 1024), kk * 2048), idesc_dq, kk ? 1u : 0u);
         umma_commit(dq_full);
         umma_commit(pds_empty);
         umma_commit(&q_empty[s]);

@@ -160,7 +160,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
   if (warp == 9) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_q);
       tma_prefetch_desc(&map_k);
       tma_prefetch_desc(&map_v);
@@ -198,7 +198,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
   } else if (warp == 8) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(128, FA_BN, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, 0, 1);
       // Two cursors over the same flattened (tile, K/V block) sequence: `a` issues S = Q K^T, `b` issues O = P V one
@@ -228,8 +228,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             umma_ss(tmem_base + TM_S + s * 128,
-                    make_smem_desc_sw128(q_base + ch * 16384 + k * 32, 16, 1024),
-                    make_smem_desc_sw128(k_base + ch * 16384 + k * 32, 16, 1024), idesc_qk,
+                    desc_at(make_smem_desc_sw128(q_base, 16, 1024), ch * 16384 + k * 32),
+                    desc_at(make_smem_desc_sw128(k_base, 16, 1024), ch * 16384 + k * 32), idesc_qk,
                     (ch | k) ? 1u : 0u);
         umma_commit(&s_full[s]);
         umma_commit(&k_empty[s]);
@@ -255,7 +255,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 #pragma unroll
         for (int kk = 0; kk < FA_BN / 16; ++kk)
           umma_ts(tmem_base + TM_O, tmem_base + TM_P + s * 64 + kk * 8,
-                  make_smem_desc_sw128(v_base + kk * 2048, 16384, 1024), idesc_pv, kk ? 1u : 0u);
+                  desc_at(make_smem_desc_sw128(v_base, 16384, 1024), kk * 2048), idesc_pv, kk ? 1u : 0u);
         umma_commit(o_full);
         umma_commit(&v_empty[s]);
         advance(bcur);

@@ -540,7 +540,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&map_a);
       tma_prefetch_desc(&map_b);
       int s = 0;
@@ -649,8 +649,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MAJOR, B_MAJOR);
+      const uint64_t adesc0 = make_smem_desc_sw128(smem_u32(smem), A_MAJOR == 0 ? 16 : 64 * BK * 2, 1024);
+      const uint64_t bdesc0 = make_smem_desc_sw128(smem_u32(smem) + A_TILE_BYTES, B_MAJOR == 0 ? 16 : 64 * BK * 2, 1024);
       int s = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -672,18 +674,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(&full[s], phase, abort_flag, p.status, TB_ERR_WAIT_FULL);
           tc_fence_after();
-          const uint32_t a_base = smem_u32(smem + s * L::STAGE_BYTES);
-          const uint32_t b_base = a_base + A_TILE_BYTES;
+          const uint64_t adesc = desc_at(adesc0, s * L::STAGE_BYTES), bdesc = desc_at(bdesc0, s * L::STAGE_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = (A_MAJOR == 0)
-                                       ? make_smem_desc_sw128(a_base + k * 32, 16, 1024)
-                                       : make_smem_desc_sw128(a_base + k * 2048, 64 * BK * 2, 1024);
-            const uint64_t bdesc = (B_MAJOR == 0)
-                                       ? make_smem_desc_sw128(b_base + k * 32, 16, 1024)
-                                       : make_smem_desc_sw128(b_base + k * 2048, 64 * BK * 2, 1024);
-            umma_ss(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k)
+            umma_ss(d_tmem, desc_at(adesc, k * (A_MAJOR == 0 ? 32 : 2048)), desc_at(bdesc, k * (B_MAJOR == 0 ? 32 : 2048)), idesc,
+                    (kb > kb0 || k > 0) ? 1u : 0u);
           umma_commit(&empty[s]);
           if (++s == STAGES) {
             s = 0;

@@ -39,6 +39,10 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
+// True in one lane of a converged warp. The thread that issues tcgen05.mma is chosen with this and not with a test of the
+// lane number: the compiler then knows that a single thread is active and feeds the uniform operands of the MMA directly;
+// with `lane == 0` an MMA took about 128 clocks to issue whatever its size (128 x 64 x 16: 0.26 us per 64-wide K block,
+// 0.16 us with elect).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -250,6 +254,9 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
   d |= (uint64_t)2 << 61;
   return d;
 }
+// The descriptor of the same matrix `bytes` further on in shared memory (addresses stay below 256 KB: the 14-bit address
+// field never carries). One add, where building the descriptor anew costs a chain of masks and shifts per MMA.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
 // Instruction descriptor for kind::f16 with bf16 inputs, fp32 accumulate.
 //   a_major / b_major: 0 = K-major, 1 = MN-major.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int a_major, int b_major) {
