@@ -16,7 +16,9 @@
 // unwired cuBLAS call (crates/torsh-backend/src/cuda/backend.rs:695-726).
 #include "comm.cuh"
 #include "fsdp_gather.cuh"
+#include "gemm_pair.cuh"
 #include "host_util.h"
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -29,18 +31,6 @@ constexpr int BK = 64;
 constexpr int A_TILE_BYTES = BM * BK * 2;
 constexpr int GEMM_THREADS = 192;
 constexpr int SCHED_DEPTH = 4;   // work indices the producer may publish ahead of the slowest consumer role
-
-enum : int {
-  EPI_BIAS = 1,          // += bias[n] (bf16)
-  EPI_GELU = 2,          // tanh-GELU after bias
-  EPI_RESIDUAL = 4,      // += residual[m,n] (bf16) after activation
-  EPI_OUT_F32 = 8,       // D is fp32 (default bf16)
-  EPI_ATOMIC = 16,       // fp32 atomic accumulate into D (split-K / grad accumulation)
-  EPI_STORE_PREACT = 32, // also store the pre-activation (after bias) as bf16
-  EPI_MUL_DGELU = 64,    // *= gelu'(aux[m,n]) (aux = forward pre-activation, bf16)
-  EPI_ACCUM = 128,       // D = D + result (non-atomic read-modify-write)
-  EPI_RASTER_M = 256,    // walk tiles with m fastest (B panel shared by concurrent CTAs)
-};
 
 struct GemmParams {
   int M, N, K;
@@ -987,11 +977,54 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
                          const void* residual, int ldr, void* preact, const void* aux, int flags,
                          int split_k, int bn, int* status, cudaStream_t stream, const TpFusion& tp);
 
+// Which kernel runs a plain product: the one of this file, CTA pairs on 256 x 256 tiles, or 128-row tiles with K split
+// over a cluster. The choice is the smallest of three modelled times (microseconds), fitted to measurements on an idle
+// B200 (fwd M x N x K: this kernel at its better width / pair / best split; cuBLAS is not involved):
+//   8192 x 4096 x 1024   58.7 / 55.2 / -         2048 x 4096 x 1024   20.8 / 18.4 / 40
+//   8192 x 1024 x 4096   58.0 / 53.2 / -         2048 x 1024 x 4096   20.5 / 26.0 / 21
+//   dgrad 2048 x 4096 x 22016  363 / 255 / -     1024 x 1024 x 4096   19.8 / 24.9 / 15.9
+//   13 x 1024 x 4096     18.8 / 23.0 / 6.9       256 x 1024 x 1024     9.5 / 10.6 / 6.5
+//   4096 x 1024 x 200     9.1 / 8.3 / -          1280 x 5120 x 104    11.4 / 12.3 / -
+// A pair needs 0.30 us per 64-wide K block of a wave of 74 tiles and at least 2.9 us for a wave's epilogue; this kernel
+// 0.25 us per K block of a wave of 148 tiles of 128 x 128 and at least 1.9 us.
+enum : int { ROUTE_ONE = 0, ROUTE_PAIR = 1 };
+
+static int route(const GemmArgs& a) {
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || !a.A || !a.B || !a.D || (a.lda & 7) || (a.ldb & 7)) return ROUTE_ONE;  // refused there
+  if (((a.flags & EPI_BIAS) && !a.bias) || ((a.flags & EPI_RESIDUAL) && !a.residual) || ((a.flags & EPI_STORE_PREACT) && !a.preact) ||
+      ((a.flags & EPI_MUL_DGELU) && !a.aux) || (a.split_k > 1 && !(a.flags & EPI_ATOMIC)))
+    return ROUTE_ONE;
+  const bool pair = gemm_pair_ok(a);
+  if (a.split_k > 1) return pair ? ROUTE_PAIR : ROUTE_ONE;  // the caller has dealt K itself
+  const long kb = (a.K + BK - 1) / BK, sms = sm_count();
+  auto waves = [](long n, long per) { return (double)((n + per - 1) / per); };
+  const double mn = a.b_major ? 1.1 : 1.0;  // MN-major B costs the one-CTA MMAs about a tenth
+  const long t256 = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
+  const long m128 = (a.M + 127) / 128, t128 = m128 * ((a.N + 127) / 128);
+  int best = ROUTE_ONE;
+  double t = 5.0 + waves(t128, sms) * fmax(kb * 0.25 * mn, 1.9);
+  if (pair) {
+    const double tp = 5.3 + waves(t256, sms / 2) * fmax(kb * 0.30 + 0.6, 2.9);
+    if (tp < t) {
+      t = tp;
+      best = ROUTE_PAIR;
+    }
+  }
+  return best;
+}
+
 TB_EXPORT int tb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int a_major,
                            int b_major, int lda, int ldb, int ldd, const void* bias,
                            const void* residual, int ldr, void* preact, const void* aux, int flags,
                            int split_k, int bn, int* status, cudaStream_t stream) {
   TB_ENSURE_DEVICE();
+  GemmArgs ga{A, B, D, M, N, K, a_major, b_major, lda, ldb, ldd, bias, residual, ldr, preact, aux, flags, split_k, status};
+  if (bn == 0 && split_k >= 0 && !g_dynamic_tiles) {
+    switch (route(ga)) {
+      case ROUTE_PAIR: return gemm_pair_launch(ga, stream);
+      default: bn = 0;
+    }
+  }
   return gemm_dispatch(A, B, D, M, N, K, a_major, b_major, lda, ldb, ldd, bias, residual, ldr, preact, aux, flags,
                        split_k, bn, status, stream, TpFusion{});
 }

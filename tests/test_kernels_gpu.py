@@ -112,6 +112,39 @@ def test_gemm_stream_k_matches_fp32(shape, majors):
     assert _rel_elem(g, ref + bias.float()) < 1e-4
 
 
+@pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("shape", [(8192, 1024, 200), (4104, 1032, 520), (2048, 4096, 64), (16400, 264, 72), (600, 50304, 128)])
+def test_gemm_pair_tiles_and_epilogues(shape, majors):
+    """Products that run on CTA pairs (256 x 256 tiles): whole and ragged tiles, one K block and several, every epilogue.
+    bf16 outputs carry one rounding (2^-9 of the element); fp32 sums of K products of N(0, 1) values in another order differ
+    by about sqrt(K) * 2^-24 * sqrt(K), well below 1e-4 of their rms."""
+    from torsh_b200 import _native as nv
+    from torsh_b200.ops.gemm import gemm
+    torch.manual_seed(11)
+    M, N, K = shape
+    am, bm = majors
+    a = torch.randn((K, M) if am else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if bm else (N, K), device=DEV, dtype=torch.bfloat16) / K ** 0.5
+    bias, res = torch.randn(N, device=DEV, dtype=torch.bfloat16), torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    pre = torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    kw = dict(a_major=am, b_major=bm)
+    u = (a.float().t() if am else a.float()) @ (b.float() if bm else b.float().t())
+    assert _rel_elem(gemm(a, b, **kw), u) < 1e-2
+    assert _rel_elem(gemm(a, b, bias=bias, residual=res, **kw), u + bias.float() + res.float()) < 1e-2
+    out = gemm(a, b, bias=bias, gelu=True, preact_out=pre, **kw)
+    assert _rel_elem(pre, u + bias.float()) < 1e-2
+    assert _rel_elem(out, torch.nn.functional.gelu(u + bias.float(), approximate="tanh")) < 1e-2
+    p = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(p, approximate="tanh").sum().backward()
+    assert _rel_elem(gemm(a, b, dgelu_aux=pre, **kw), u * p.grad) < 1e-2
+    g = torch.ones(M, N, device=DEV)
+    gemm(a, b, out=g, atomic=True, split_k=min(3, (K + 63) // 64), bias=bias, **kw)
+    assert _rel_elem(g, u + 1.0 + bias.float()) < 1e-4
+    gemm(a, b, out=g, **kw)
+    assert _rel_elem(g, u) < 1e-4
+    nv.check_status()
+
+
 # ------------------------------------------------------------------ norms
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [256, 1024, 4096])

@@ -41,12 +41,32 @@ def _wgrad_plan(m_out: int, n_out: int, k: int) -> tuple[int, int]:
     return bn, sk
 
 
+def _wgrad_pair_split(m_out: int, n_out: int, k: int, accumulate: bool) -> int:
+    """Split-K factor of a weight-gradient GEMM on CTA pairs (outputs of at least one 256 x 256 tile).
+
+    A piece of K costs its K-blocks plus about ten more for filling and draining, and there are 74 pairs, so the smallest
+    ``waves * (kb / sk + 10)`` wins. Measured at K = 8192: 64 tiles 54 / 57 / 60 us with 1 / 2 / 3 splits, 48 tiles 50 / 54 /
+    44, 16 tiles 50 / 31 / 25 and 21 with 4 (one-CTA kernel with its best plan: 70, 59, 32). Without an fp32 buffer to
+    accumulate into, splits also pay for making one and casting it: two launches and 10 bytes an element, in K-blocks of
+    0.3 us."""
+    kb = (k + 63) // 64
+    tiles = ((m_out + 255) // 256) * ((n_out + 255) // 256)
+    extra = 0.0 if accumulate else 40.0 + m_out * n_out / 3e5
+
+    def cost(sk):
+        return -(-tiles * sk // 74) * (-(-kb // sk) + 10) + (extra if sk > 1 else 0.0)
+    return min(range(1, max(1, min(9, kb // 8)) + 1), key=cost)
+
+
 def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layout: str):
     """dW for y = x Wᵀ (nk) or y = x W (kn). Returns a grad tensor, or None after accumulating into main_grad."""
     a, b = (dy2, x2) if layout == "nk" else (x2, dy2)
     m_out, n_out, k = a.shape[1], b.shape[1], a.shape[0]
-    bn, sk = _wgrad_plan(m_out, n_out, k)
     mg = getattr(weight, "main_grad", None)
+    if m_out >= 256 and n_out >= 256:
+        bn, sk = 0, _wgrad_pair_split(m_out, n_out, k, mg is not None)
+    else:
+        bn, sk = _wgrad_plan(m_out, n_out, k)
     if mg is not None:
         gemm(a, b, a_major=1, b_major=1, out=mg, atomic=True, split_k=sk, bn=bn)
         return None
