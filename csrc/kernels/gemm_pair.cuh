@@ -30,7 +30,10 @@ struct GemmArgs {
 
 // True when the kernel can run this product (alignment, epilogue).
 bool gemm_pair_ok(const GemmArgs& a);
+bool gemm_split_ok(const GemmArgs& a);
 // CTA pairs on 256 x 256 tiles (gemm_pair_sm100.cu); split_k > 1 needs EPI_ATOMIC.
 int gemm_pair_launch(const GemmArgs& a, cudaStream_t stream);
+// 128 x bn tiles (bn 64 or 128), K split over a cluster of S = 1, 2, 4 or 8 CTAs (gemm_split_sm100.cu); bf16 output.
+int gemm_split_launch(const GemmArgs& a, int bn, int S, cudaStream_t stream);
 
 }  // namespace tb

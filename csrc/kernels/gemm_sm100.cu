@@ -987,9 +987,9 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
 //   4096 x 1024 x 200     9.1 / 8.3 / -          1280 x 5120 x 104    11.4 / 12.3 / -
 // A pair needs 0.30 us per 64-wide K block of a wave of 74 tiles and at least 2.9 us for a wave's epilogue; this kernel
 // 0.25 us per K block of a wave of 148 tiles of 128 x 128 and at least 1.9 us.
-enum : int { ROUTE_ONE = 0, ROUTE_PAIR = 1 };
+enum : int { ROUTE_ONE = 0, ROUTE_PAIR = 1, ROUTE_SPLIT = 2 };
 
-static int route(const GemmArgs& a) {
+static int route(const GemmArgs& a, int& bn, int& S) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || !a.A || !a.B || !a.D || (a.lda & 7) || (a.ldb & 7)) return ROUTE_ONE;  // refused there
   if (((a.flags & EPI_BIAS) && !a.bias) || ((a.flags & EPI_RESIDUAL) && !a.residual) || ((a.flags & EPI_STORE_PREACT) && !a.preact) ||
       ((a.flags & EPI_MUL_DGELU) && !a.aux) || (a.split_k > 1 && !(a.flags & EPI_ATOMIC)))
@@ -1010,6 +1010,25 @@ static int route(const GemmArgs& a) {
       best = ROUTE_PAIR;
     }
   }
+  // A split CTA needs 0.18 (64 wide) or 0.25 us per K block, 0.6 us for the exchange and 3.5 us for every further wave, whose
+  // prologue nothing hides. Clusters of 4 and 8 do not fill every GPC: 120 and 112 CTAs at a time were seen on 148 SMs.
+  if (sms >= 128 && gemm_split_ok(a)) {
+    for (int w = 64; w <= 128; w *= 2) {
+      const long tiles = m128 * ((a.N + w - 1) / w);
+      for (int s = 1; s <= 8 && s <= kb; s *= 2) {
+        const long cap = s <= 2 ? sms : s == 4 ? sms * 120 / 148 : sms * 112 / 148;
+        const double wv = waves(tiles * s, cap);
+        if (wv > 2) break;
+        const double ts = 5.2 + (s > 1 ? 0.6 : 0.0) + (wv - 1) * 3.5 + wv * (double)((kb + s - 1) / s) * (w == 64 ? 0.18 : 0.25) * mn;
+        if (ts < t) {
+          t = ts;
+          best = ROUTE_SPLIT;
+          bn = w;
+          S = s;
+        }
+      }
+    }
+  }
   return best;
 }
 
@@ -1020,8 +1039,10 @@ TB_EXPORT int tb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, 
   TB_ENSURE_DEVICE();
   GemmArgs ga{A, B, D, M, N, K, a_major, b_major, lda, ldb, ldd, bias, residual, ldr, preact, aux, flags, split_k, status};
   if (bn == 0 && split_k >= 0 && !g_dynamic_tiles) {
-    switch (route(ga)) {
+    int S = 1;
+    switch (route(ga, bn, S)) {
       case ROUTE_PAIR: return gemm_pair_launch(ga, stream);
+      case ROUTE_SPLIT: return gemm_split_launch(ga, bn, S, stream);
       default: bn = 0;
     }
   }

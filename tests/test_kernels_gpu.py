@@ -145,6 +145,34 @@ def test_gemm_pair_tiles_and_epilogues(shape, majors):
     nv.check_status()
 
 
+@pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("shape", [(8, 64, 128), (16, 1024, 4096), (136, 200, 4160), (512, 1024, 4096), (264, 1608, 520)])
+def test_gemm_cluster_split_k(shape, majors):
+    """Small products, K split over a cluster: remainders of rows, columns and K blocks, every epilogue of a bf16 output.
+    The outputs carry one rounding (2^-9 of the element) and are the same in every run (the partial sums have an order)."""
+    from torsh_b200 import _native as nv
+    from torsh_b200.ops.gemm import gemm
+    torch.manual_seed(12)
+    M, N, K = shape
+    am, bm = majors
+    a = torch.randn((K, M) if am else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if bm else (N, K), device=DEV, dtype=torch.bfloat16) / K ** 0.5
+    bias, res = torch.randn(N, device=DEV, dtype=torch.bfloat16), torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    pre = torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    kw = dict(a_major=am, b_major=bm)
+    u = (a.float().t() if am else a.float()) @ (b.float() if bm else b.float().t())
+    out = gemm(a, b, **kw)
+    assert _rel_elem(out, u) < 1e-2 and torch.equal(out, gemm(a, b, **kw))
+    v = u + bias.float()
+    out = gemm(a, b, bias=bias, gelu=True, residual=res, preact_out=pre, **kw)
+    assert _rel_elem(pre, v) < 1e-2
+    assert _rel_elem(out, torch.nn.functional.gelu(v, approximate="tanh") + res.float()) < 1e-2
+    p = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(p, approximate="tanh").sum().backward()
+    assert _rel_elem(gemm(a, b, dgelu_aux=pre, **kw), u * p.grad) < 1e-2
+    nv.check_status()
+
+
 # ------------------------------------------------------------------ norms
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [256, 1024, 4096])
