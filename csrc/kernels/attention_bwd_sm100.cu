@@ -4,7 +4,7 @@
 //   S  = Q_i K_j^T          dP = dO_i V_j^T                   (tensor core, into TMEM)
 //   P  = exp(S*scale - L_i) dS = P * (dP - delta_i) * scale   (compute warps, fp32)
 //   dV_j += P^T dO_i        dK_j += dS^T Q_i                  (accumulate in TMEM over i)
-//   dQ_i += dS K_j                                            (TMEM -> fp32 atomics in global)
+//   dQ_i += dS K_j                                            (TMEM -> shared memory -> bulk fp32 reduce-add in global)
 // P and dS are written by the compute warps into shared memory in the 128-byte-swizzled layout
 // that tcgen05.mma descriptors read, once, and that one buffer serves both as the K-major A
 // operand (dQ) and as the MN-major A operand (dK, dV) - no transposes anywhere. Q, dO, K, V tiles
@@ -25,7 +25,7 @@ constexpr int FB_THREADS = 320;  // 8 compute warps + MMA warp + TMA warp
 struct FaBwdParams {
   const float* LSE;    // [B, H, S]
   const float* delta;  // [B, H, S]  rowsum(dO * O)
-  float* dQ_acc;       // fp32 [B*S, H*D] accumulated with atomics
+  float* dQ_acc;       // fp32, accumulated: [B*H][query blocks][D / 32][128 rows][32 columns, 16-byte chunks xor row % 8]
   __nv_bfloat16* dK;   // [B*S, dkv_stride], head h at column h*D
   __nv_bfloat16* dV;
   int B, S, H;
@@ -45,7 +45,8 @@ struct FaBwdSmem {
   static constexpr int DO_OFF = Q_OFF + QST * TILE;
   static constexpr int P_OFF = DO_OFF + QST * TILE;
   static constexpr int DS_OFF = P_OFF + 32768;
-  static constexpr int BAR_OFF = DS_OFF + 32768;
+  static constexpr int DQ_OFF = DS_OFF + 32768;  // per compute warp: 32 rows x 32 fp32 columns of dQ on their way out
+  static constexpr int BAR_OFF = DQ_OFF + 8 * 4096;
   // kv_full, q_full[2], q_empty[2], do_full[2], do_empty[2], s_full, dp_full, ds_full,
   // pds_empty, dq_full, dq_empty, dkv_full, s_free, dp_free
   static constexpr int NBARS = 18;
@@ -272,25 +273,32 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     uint8_t* p_smem = smem + L::P_OFF;
     uint8_t* ds_smem = smem + L::DS_OFF;
     const int sw = row & 7;
-    // dQ partial of query block tt: TMEM -> fp32 reductions into the global accumulator
+    // dQ partial of query block tt: TMEM -> this warp's staging rows -> one 4 KB bulk reduce-add per 32 columns. The
+    // accumulator keeps the staged order (the cast pass undoes it), so that a warp's rows are one contiguous run: as
+    // 16-byte reductions of every lane into its own row they reached 1.1 to 1.5 TB/s of L2 and bounded the kernel.
+    uint8_t* dq_stage = smem + L::DQ_OFF + warp * 4096;
     auto drain_dq = [&](int tt) {
-      const int qd = (i0 + tt) * 128 + row;
-      const bool ok = qd < p.S;
       mbar_wait(dq_full, tt & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
-      float* dq_row = p.dQ_acc + ((size_t)b * p.S + (ok ? qd : 0)) * ((size_t)p.H * D) + (size_t)h * D;
+      float* dq_blk = p.dQ_acc + (((size_t)bh * n_blk + i0 + tt) * (D / 32)) * 4096 + (warp & 3) * 1024;
 #pragma unroll 1
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
         uint32_t v[32];
         tmem_ld32(tmem_base + TM_DQ + c * 32 + lane_off, v);
         tmem_wait_ld();
-        if (ok) {
+        if (lane == 0) bulk_wait_read_all();  // the previous run has left the staging rows
+        __syncwarp();
 #pragma unroll
-          for (int g = 0; g < 8; ++g)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dq_row + c * 32 + g * 4),
-                         "f"(__uint_as_float(v[g * 4])), "f"(__uint_as_float(v[g * 4 + 1])),
-                         "f"(__uint_as_float(v[g * 4 + 2])), "f"(__uint_as_float(v[g * 4 + 3]))
-                         : "memory");
+        for (int g = 0; g < 8; ++g)
+          *reinterpret_cast<uint4*>(dq_stage + lane * 128 + ((g ^ sw) << 4)) =
+              make_uint4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_blk + c * 4096),
+                       "r"(smem_u32(dq_stage)), "r"(4096)
+                       : "memory");
+          bulk_commit();
         }
       }
       tc_fence_before();
@@ -353,6 +361,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       }
     }
     if (PIPELINED && n_it > 0) drain_dq(n_it - 1);
+    if (lane == 0) bulk_wait_all();
     // dK, dV of this key block: thread = key row
     mbar_wait(dkv_full, 0, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
     tc_fence_after();
@@ -423,19 +432,24 @@ __global__ void fa_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_
   }
 }
 
-// dst[t, col0 + c] = bf16(src[t, c]) for c < cols (fp32 accumulator -> strided bf16 gradient)
-__global__ void fa_cvt_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long rows,
-                                 int cols, long dst_stride) {
-  const long total = rows * (cols / 4);
+// dQ: the fp32 accumulator's blocks (layout at FaBwdParams::dQ_acc) -> bf16 rows. One thread per 8 columns of a row.
+__global__ void fa_cvt_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int B, int S, int H, int D,
+                                 int n_blk, long dst_stride) {
+  const int vpr = D / 8;  // vectors per (token, head)
+  const long total = (long)B * S * H * vpr;
   const long stride = (long)gridDim.x * blockDim.x;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-    long r = idx / (cols / 4);
-    int c = (int)(idx - r * (cols / 4)) * 4;
-    float4 v = *reinterpret_cast<const float4*>(src + r * cols + c);
-    uint2 o;
-    o.x = pack_bf16x2(v.x, v.y);
-    o.y = pack_bf16x2(v.z, v.w);
-    *reinterpret_cast<uint2*>(dst + r * dst_stride + c) = o;
+    const int v = (int)(idx % vpr);
+    const long th = idx / vpr;
+    const int h = (int)(th % H);
+    const long tok = th / H;
+    const int b = (int)(tok / S), s = (int)(tok - (long)b * S);
+    const int row = s & 127, c = v >> 2, g = (v & 3) * 2;
+    const float* blk = src + ((((size_t)b * H + h) * n_blk + (s >> 7)) * (D / 32) + c) * 4096 + row * 32;
+    const float4 x = *reinterpret_cast<const float4*>(blk + ((g ^ (row & 7)) << 2));
+    const float4 y = *reinterpret_cast<const float4*>(blk + (((g + 1) ^ (row & 7)) << 2));
+    *reinterpret_cast<uint4*>(dst + tok * dst_stride + (long)h * D + v * 8) =
+        make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
   }
 }
 
@@ -449,7 +463,7 @@ inline int make_bshd_map_bwd(CUtensorMap* m, const void* base, int B, int S, int
 }  // namespace tb
 using namespace tb;
 
-// Workspace (caller-provided): delta fp32 [B*H*S], dq_acc fp32 [B*S*H*D] (zeroed here).
+// Workspace (caller-provided, 16-byte aligned): delta fp32 [B*H*S], dq_acc fp32 [B*H*ceil(S/128)*128*D] (zeroed here).
 // dq, dk, dv: bf16 [B*S, dqkv_stride] with head h at column h*D (may be the three column bands of
 // one fused dQKV buffer).
 TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
@@ -476,7 +490,7 @@ TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, con
     fa_delta_kernel<64><<<(unsigned)((nthreads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_stride, do_stride);
   else
     fa_delta_kernel<128><<<(unsigned)((nthreads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_stride, do_stride);
-  TB_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * S * H * D, st));
+  TB_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * H * ((S + 127) / 128) * 128 * D, st));
   FaBwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, B, S, H, dqkv_stride, scale, causal, status};
   const int n_blk = (S + 127) / 128;
   const long grid = (long)n_blk * B * H;
@@ -489,10 +503,9 @@ TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, con
     if (!cfg) { TB_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaBwdSmem<128>::ALLOC)); cfg = true; }
     fa_bwd_kernel<128><<<(unsigned)grid, FB_THREADS, FaBwdSmem<128>::ALLOC, st>>>(mq, mk, mv, mdo, p);
   }
-  const long rows = (long)B * S;
-  long items = rows * (H * D / 4);
+  const long items = (long)B * S * H * (D / 8);
   int g = (int)((items + 255) / 256 < (long)sm_count() * 16 ? (items + 255) / 256 : (long)sm_count() * 16);
-  fa_cvt_dq_kernel<<<g, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, rows, H * D, dqkv_stride);
+  fa_cvt_dq_kernel<<<g, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, B, S, H, D, n_blk, dqkv_stride);
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
