@@ -1,17 +1,28 @@
 // Flash attention backward for sm_100a (tcgen05 / TMEM / TMA), causal or full, head dim 64 / 128.
 //
-// One CTA per (batch, head, 128-key block); it walks the query blocks that see those keys:
-//   S  = Q_i K_j^T          dP = dO_i V_j^T                   (tensor core, into TMEM)
-//   P  = exp(S*scale - L_i) dS = P * (dP - delta_i) * scale   (compute warps, fp32)
-//   dV_j += P^T dO_i        dK_j += dS^T Q_i                  (accumulate in TMEM over i)
-//   dQ_i += dS K_j                                            (TMEM -> shared memory -> bulk fp32 reduce-add in global)
-// P and dS are written by the compute warps into shared memory in the 128-byte-swizzled layout
-// that tcgen05.mma descriptors read, once, and that one buffer serves both as the K-major A
-// operand (dQ) and as the MN-major A operand (dK, dV) - no transposes anywhere. Q, dO, K, V tiles
-// are the TMA-loaded tiles themselves, used K-major or MN-major as each product needs.
-// TMEM: S | dP (128 cols each) | dV | dK (D each) | dQ partial (D; aliases S when D = 128).
-// Warps 0-7 compute (two threads per query row = TMEM lane, each owning half of the columns), warp 8
-// issues MMAs, warp 9 drives TMA.
+// One CTA per (batch, head, 128-key block); it walks the query blocks that see those keys. Scores are kept transposed
+// (TMEM lane = key), so that P^T is a tensor-memory operand and never goes through shared memory:
+//   S^T  = K_j Q_i^T         dP^T = V_j dO_i^T                   (tensor core, into TMEM)
+//   P^T  = exp(S^T*scale - L_i)  dS^T = P^T * (dP^T - delta_i) * scale   (compute warps, fp32)
+//   dV_j += P^T dO_i         dK_j += dS^T Q_i                    (accumulate in TMEM over i)
+//   dQ_i += dS K_j                                               (TMEM -> shared memory -> bulk fp32 reduce-add in global)
+// dS^T goes to shared memory once, in the 128-byte-swizzled layout of the MMA
+// descriptors, and serves as the K-major A operand of dK and as the MN-major A operand of dQ.
+//
+// What bounds it is the chain of a query block (scores, exponentials, dP, dS, three products, dQ out), so the chain is cut
+// into roles that work on different blocks at the same time. 16 warps:
+//   warps 0-7    compute, two threads per key row, each owning 64 queries of the block
+//   warps 8-11   dQ out: drain block t while the compute warps evaluate the exponentials of block t + 1
+//   warp 12      MMA issuer: the scores of block t + 1 go out as soon as block t has left their columns
+//   warp 13      TMA producer (Q two blocks deep, dO one);  warp 14  L and delta rows into a two-deep ring
+// TMEM: S^T | dP^T (128 columns each) | dV | dK (D each), and with D = 64 dQ | P^T (64 each).
+// Registers are moved between the warpgroups with setmaxnreg: 512 threads x 128 at launch, 160 for the two compute groups,
+// 88 and 104 for the others.
+// One role after the other per block (P and dS both through shared memory) took 633 us where this takes 400 with everything
+// around it (B2 S4096 H16 D128 causal), 214 where this takes 136 (B1 S2048 H32 D128), and 129 where this takes 117
+// (B8 S1024 H16 D64). What bounds it now with D = 64 is shared memory: about 3400 clocks of 128 bytes per block for the MMA
+// operands, the L and delta broadcasts, dS and dQ, against 1300 clocks of MMA and 1024 of exponentials. Four compute threads
+// per row instead of two and conversions on the FMA pipe changed nothing.
 //
 // The reference has no attention backward at all (its autograd tape covers only
 // add/sub/mul/matmul/pow/mean/sum: crates/torsh-tensor/src/core_ops/types.rs:1497-1658).
@@ -20,7 +31,7 @@
 
 namespace tb {
 
-constexpr int FB_THREADS = 320;  // 8 compute warps + MMA warp + TMA warp
+constexpr int FB_THREADS = 512;
 
 struct FaBwdParams {
   const float* LSE;    // [B, H, S]
@@ -38,43 +49,60 @@ struct FaBwdParams {
 template <int D>
 struct FaBwdSmem {
   static constexpr int TILE = 128 * D * 2;
-  static constexpr int QST = (D == 64) ? 2 : 1;  // Q / dO ring depth
+  static constexpr int DOST = (D == 64) ? 2 : 1;  // dO ring depth
   static constexpr int K_OFF = 0;
   static constexpr int V_OFF = TILE;
   static constexpr int Q_OFF = 2 * TILE;
-  static constexpr int DO_OFF = Q_OFF + QST * TILE;
-  static constexpr int P_OFF = DO_OFF + QST * TILE;
-  static constexpr int DS_OFF = P_OFF + 32768;
-  static constexpr int DQ_OFF = DS_OFF + 32768;  // per compute warp: 32 rows x 32 fp32 columns of dQ on their way out
-  static constexpr int BAR_OFF = DQ_OFF + 8 * 4096;
-  // kv_full, q_full[2], q_empty[2], do_full[2], do_empty[2], s_full, dp_full, ds_full,
-  // pds_empty, dq_full, dq_empty, dkv_full, s_free, dp_free
-  static constexpr int NBARS = 18;
-  static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16;
-  static constexpr int ALLOC = TOTAL + 1024;
+  static constexpr int DO_OFF = Q_OFF + 2 * TILE;
+  static constexpr int DS_OFF = DO_OFF + DOST * TILE;
+  static constexpr int DQ_OFF = DS_OFF + 32768;        // per dQ warp: 2 x (32 rows x 32 fp32 columns) on their way out
+  static constexpr int LD_OFF = DQ_OFF + 4 * 8192;     // -L * log2(e) and -delta * scale of a query block, 2 stages
+  static constexpr int BAR_OFF = LD_OFF + 2 * 2 * 512;
+  // kv_full, q_full[2], q_empty[2], do_full[2], do_empty[2], ld_full[2], ld_empty[2], s_full, p_full, dp_full, ds_full,
+  // ds_empty, dv_done, dq_full, dq_empty, dkv_full
+  static constexpr int NBARS = 22;
+  static constexpr int ALLOC = BAR_OFF + NBARS * 8 + 16;
+  static_assert(ALLOC <= 232448, "shared memory budget of one CTA exceeded");
 };
 
-// P = exp2(S * sl2 - L) and dS = P * (dP - delta) * scale for 32 scores of one row, both packed to bf16 pairs. The
-// scale-and-shift steps run as packed two-wide fp32 instructions; MASK is a template parameter so that blocks away from
-// the diagonal and the ragged edge carry no compare / select instructions.
+// e = exp2(S^T * sl2 - L) for 32 queries of one key row, and the same packed to bf16 pairs. `first` is the first query (as
+// an index of this call's 32) that sees the key; MASK is a template parameter so that blocks away from the diagonal and the
+// ragged edge carry no compare / select instructions. --L comes from shared memory (the same for every lane: broadcast).
 template <bool MASK>
-__device__ __forceinline__ void fa_bwd_p_ds(const uint32_t (&sv)[32], const uint32_t (&dv)[32], float sl2, float Lr,
-                                            float scale, float dr, int kvbase, int col_limit, uint32_t (&pp)[16],
-                                            uint32_t (&dd)[16]) {
-  const float2 s2 = make_float2(sl2, sl2), l2 = make_float2(-Lr, -Lr);
-  const float2 c2 = make_float2(scale, scale), d2 = make_float2(-dr * scale, -dr * scale);
+__device__ __forceinline__ void fa_bwd_p(const uint32_t (&sv)[32], const float* L, float sl2, int first, float (&e)[32],
+                                         uint32_t (&pk)[16]) {
+  const float2 s2 = make_float2(sl2, sl2);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float2 t = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), s2, l2);
-    float2 e = make_float2(exp2f(t.x), exp2f(t.y));
+  for (int i = 0; i < 32; i += 4) {
+    const float4 l4 = *reinterpret_cast<const float4*>(L + i);
+    const float2 t0 = __ffma2_rn(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), s2, make_float2(l4.x, l4.y));
+    const float2 t1 = __ffma2_rn(make_float2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])), s2, make_float2(l4.z, l4.w));
+    e[i] = exp2f(t0.x);
+    e[i + 1] = exp2f(t0.y);
+    e[i + 2] = exp2f(t1.x);
+    e[i + 3] = exp2f(t1.y);
     if (MASK) {
-      if (kvbase + 2 * i > col_limit) e.x = 0.f;
-      if (kvbase + 2 * i + 1 > col_limit) e.y = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i + j < first) e[i + j] = 0.f;
     }
-    const float2 g = __ffma2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), c2, d2);
-    const float2 ds = __fmul2_rn(e, g);
-    pp[i] = pack_bf16x2(e.x, e.y);
-    dd[i] = pack_bf16x2(ds.x, ds.y);
+    pk[i >> 1] = pack_bf16x2(e[i], e[i + 1]);
+    pk[(i >> 1) + 1] = pack_bf16x2(e[i + 2], e[i + 3]);
+  }
+}
+
+// dS^T = e * (dP^T * scale - delta * scale) for 32 queries, packed to bf16 pairs (the ring holds -delta * scale)
+__device__ __forceinline__ void fa_bwd_ds(const uint32_t (&dv)[32], const float* ds_row, float scale, const float (&e)[32],
+                                          uint32_t (&dd)[16]) {
+  const float2 c2 = make_float2(scale, scale);
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    const float4 d4 = *reinterpret_cast<const float4*>(ds_row + i);
+    const float2 g0 = __ffma2_rn(make_float2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), c2, make_float2(d4.x, d4.y));
+    const float2 g1 = __ffma2_rn(make_float2(__uint_as_float(dv[i + 2]), __uint_as_float(dv[i + 3])), c2, make_float2(d4.z, d4.w));
+    const float2 a = __fmul2_rn(make_float2(e[i], e[i + 1]), g0), b = __fmul2_rn(make_float2(e[i + 2], e[i + 3]), g1);
+    dd[i >> 1] = pack_bf16x2(a.x, a.y);
+    dd[(i >> 1) + 1] = pack_bf16x2(b.x, b.y);
   }
 }
 
@@ -85,39 +113,40 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
               const FaBwdParams p) {
   using L = FaBwdSmem<D>;
   constexpr int KCH = D / 64;
-  constexpr int QST = L::QST;
+  constexpr int DOST = L::DOST;
   constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = 256 + D;
-  constexpr uint32_t TM_DQ = (D == 64) ? 384 : 0;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  // With D = 64 there is room for P^T and dQ beside the rest, and the scores of the next block can be issued early. With
+  // D = 128 P^T takes the first half of the S^T columns it came from (a compute half's 64 queries: 32 of its 64 columns)
+  // and dQ the columns of dP^T once they have been read.
+  constexpr bool ROOMY = D == 64;
+  constexpr uint32_t TM_DQ = ROOMY ? 384 : TM_DP;
+  constexpr uint32_t TM_P = ROOMY ? 448 : TM_S, P_HALF = ROOMY ? 32 : 64;
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;
   uint64_t* q_empty = bars + 3;
   uint64_t* do_full = bars + 5;
   uint64_t* do_empty = bars + 7;
-  uint64_t* s_full = bars + 9;
-  uint64_t* dp_full = bars + 10;
-  uint64_t* ds_full = bars + 11;
-  uint64_t* pds_empty = bars + 12;
-  uint64_t* dq_full = bars + 13;
-  uint64_t* dq_empty = bars + 14;
-  uint64_t* dkv_full = bars + 15;
-  uint64_t* s_free = bars + 16;    // compute warps have read S of the current block out of TMEM (head dim 64 only)
-  uint64_t* dp_free = bars + 17;   // ... and dP
-  // Head dim 64 runs software-pipelined: the score MMAs of query block t + 1 are issued as soon as the compute warps
-  // have copied S[t] / dP[t] into registers, so the tensor core works on block t + 1 while they evaluate the
-  // exponentials of block t, and the dQ partial of block t is drained (TMEM -> fp32 reductions) after the compute of
-  // block t + 1, when its MMAs have long finished. With head dim 128 dQ shares TMEM columns with S, which forbids the
-  // early issue, and the blocks run one after the other.
-  constexpr bool PIPELINED = (D == 64);
+  uint64_t* ld_full = bars + 9;
+  uint64_t* ld_empty = bars + 11;
+  uint64_t* s_full = bars + 13;    // S^T[t] is in TMEM
+  uint64_t* p_full = bars + 14;    // P^T[t] has replaced it
+  uint64_t* dp_full = bars + 15;   // dP^T[t] is in TMEM
+  uint64_t* ds_full = bars + 16;   // dP^T[t] has been read, dS^T[t] is in shared memory
+  uint64_t* ds_empty = bars + 17;  // dK and dQ of block t have read dS^T[t]
+  uint64_t* dv_done = bars + 18;   // dV of block t has read P^T[t]
+  uint64_t* dq_full = bars + 19;   // dQ partial of block t is in TMEM
+  uint64_t* dq_empty = bars + 20;  // ... and has been read
+  uint64_t* dkv_full = bars + 21;
   uint32_t* tmem_ptr = (uint32_t*)(bars + L::NBARS);
   volatile int* abort_flag = (volatile int*)(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_blk = (p.S + 127) / 128;
-  const int jb = blockIdx.x % n_blk;  // key block; early key blocks (most work when causal) first
-  const int bh = blockIdx.x / n_blk;
+  const int BH = p.B * p.H;
+  const int jb = blockIdx.x / BH;     // key block; the early key blocks of all heads first: with a causal mask they are the long ones
+  const int bh = blockIdx.x - jb * BH;
   const int h = bh % p.H, b = bh / p.H;
   const int kv0 = jb * 128;
   const int i0 = p.causal ? jb : 0;
@@ -130,20 +159,24 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       mbar_init(&q_empty[i], 1);
       mbar_init(&do_full[i], 1);
       mbar_init(&do_empty[i], 1);
+      mbar_init(&ld_full[i], 32);
+      mbar_init(&ld_empty[i], 256);
     }
     mbar_init(s_full, 1);
+    mbar_init(p_full, 256);
     mbar_init(dp_full, 1);
     mbar_init(ds_full, 256);
-    mbar_init(pds_empty, 1);
+    mbar_init(ds_empty, 1);
+    mbar_init(dv_done, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 256);
+    mbar_init(dq_empty, 128);
     mbar_init(dkv_full, 1);
-    mbar_init(s_free, 256);
-    mbar_init(dp_free, 256);
-    *abort_flag = 0;
+    // the 128-byte swizzle needs a 1024-byte aligned window; with the flag up no role loads or waits
+    *abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;
+    if (*abort_flag && p.status) atomicCAS(p.status, 0, TB_ERR_BAD_ARG);
     fence_barrier_init();
   }
-  if (warp == 8) {
+  if (warp == 12) {
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
   }
@@ -151,224 +184,244 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
 
-  if (warp == 9) {
-    // ---------------------------------------------------------------- TMA producer
-    if (elect_one()) {
-      tma_prefetch_desc(&map_q);
-      tma_prefetch_desc(&map_k);
-      tma_prefetch_desc(&map_v);
-      tma_prefetch_desc(&map_do);
-      mbar_expect_tx(kv_full, 2 * L::TILE);
+  if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    if (warp == 13) {
+      // -------------------------------------------------------------- TMA producer
+      if (elect_one() && !*abort_flag) {
+        tma_prefetch_desc(&map_q);
+        tma_prefetch_desc(&map_k);
+        tma_prefetch_desc(&map_v);
+        tma_prefetch_desc(&map_do);
+        mbar_expect_tx(kv_full, 2 * L::TILE);
 #pragma unroll
-      for (int c = 0; c < KCH; ++c) {
-        tma_load_4d(smem + L::K_OFF + c * 16384, &map_k, kv_full, c * 64, h, kv0, b);
-        tma_load_4d(smem + L::V_OFF + c * 16384, &map_v, kv_full, c * 64, h, kv0, b);
-      }
-      for (int t = 0; t < n_it; ++t) {
-        const int s = t % QST;
-        const uint32_t ph = (t / QST) & 1;
-        const int qrow0 = (i0 + t) * 128;
-        // once a wait has given up, nothing more is loaded: loads without a free slot would pile transaction counts
-        // on one barrier beyond its range
-        if (!mbar_wait(&q_empty[s], ph ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY)) break;
-        mbar_expect_tx(&q_full[s], L::TILE);
+        for (int c = 0; c < KCH; ++c) {
+          tma_load_4d(smem + L::K_OFF + c * 16384, &map_k, kv_full, c * 64, h, kv0, b);
+          tma_load_4d(smem + L::V_OFF + c * 16384, &map_v, kv_full, c * 64, h, kv0, b);
+        }
+        for (int t = 0; t < n_it; ++t) {
+          const int s = t & 1, sd = t % DOST;
+          const int qrow0 = (i0 + t) * 128;
+          // once a wait has given up, nothing more is loaded: loads without a free slot would pile transaction counts
+          // on one barrier beyond its range
+          if (!mbar_wait(&q_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY)) break;
+          mbar_expect_tx(&q_full[s], L::TILE);
 #pragma unroll
-        for (int c = 0; c < KCH; ++c)
-          tma_load_4d(smem + L::Q_OFF + s * L::TILE + c * 16384, &map_q, &q_full[s], c * 64, h, qrow0, b);
-        if (!mbar_wait(&do_empty[s], ph ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY)) break;
-        mbar_expect_tx(&do_full[s], L::TILE);
+          for (int c = 0; c < KCH; ++c)
+            tma_load_4d(smem + L::Q_OFF + s * L::TILE + c * 16384, &map_q, &q_full[s], c * 64, h, qrow0, b);
+          if (!mbar_wait(&do_empty[sd], ((t / DOST) & 1) ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY)) break;
+          mbar_expect_tx(&do_full[sd], L::TILE);
 #pragma unroll
-        for (int c = 0; c < KCH; ++c)
-          tma_load_4d(smem + L::DO_OFF + s * L::TILE + c * 16384, &map_do, &do_full[s], c * 64, h, qrow0, b);
-      }
-      if (*abort_flag) {
-        uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 2000000ull) {
+          for (int c = 0; c < KCH; ++c)
+            tma_load_4d(smem + L::DO_OFF + sd * L::TILE + c * 16384, &map_do, &do_full[sd], c * 64, h, qrow0, b);
+        }
+        if (*abort_flag) {
+          uint64_t t0 = globaltimer_ns();
+          while (globaltimer_ns() - t0 < 2000000ull) {
+          }
         }
       }
-    }
-  } else if (warp == 8) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_dkv = make_idesc_bf16(128, D, 1, 1);
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, 0, 1);
-      const uint32_t k_base = smem_u32(smem + L::K_OFF);
-      const uint32_t v_base = smem_u32(smem + L::V_OFF);
-      const uint32_t p_base = smem_u32(smem + L::P_OFF);
-      const uint32_t ds_base = smem_u32(smem + L::DS_OFF);
-      mbar_wait(kv_full, 0, abort_flag, p.status, TB_ERR_WAIT_FULL);
-      // S = Q_t K^T and dP = dO_t V^T of query block t (each waits for its TMEM columns when pipelined)
-      auto issue_scores = [&](int t) {
-        const int s = t % QST;
-        const uint32_t ph = (t / QST) & 1;
-        const uint32_t q_base = smem_u32(smem + L::Q_OFF + s * L::TILE);
-        const uint32_t do_base = smem_u32(smem + L::DO_OFF + s * L::TILE);
-        if (PIPELINED && t > 0) mbar_wait(s_free, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
-        mbar_wait(&q_full[s], ph, abort_flag, p.status, TB_ERR_WAIT_FULL);
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < KCH; ++c)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ss(tmem_base + TM_S, desc_at(make_smem_desc_sw128(q_base, 16, 1024), c * 16384 + k * 32),
-                    desc_at(make_smem_desc_sw128(k_base, 16, 1024), c * 16384 + k * 32), idesc_s, (c | k) ? 1u : 0u);
-        umma_commit(s_full);
-        if (PIPELINED && t > 0) mbar_wait(dp_free, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
-        mbar_wait(&do_full[s], ph, abort_flag, p.status, TB_ERR_WAIT_FULL);
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < KCH; ++c)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ss(tmem_base + TM_DP, desc_at(make_smem_desc_sw128(do_base, 16, 1024), c * 16384 + k * 32),
-                    desc_at(make_smem_desc_sw128(v_base, 16, 1024), c * 16384 + k * 32), idesc_s, (c | k) ? 1u : 0u);
-        umma_commit(dp_full);
-      };
-      if (PIPELINED && n_it > 0) issue_scores(0);
+    } else if (warp == 14) {
+      // -------------------------------------------------------------- L and delta rows
       for (int t = 0; t < n_it; ++t) {
-        const int s = t % QST;
-        const uint32_t q_base = smem_u32(smem + L::Q_OFF + s * L::TILE);
-        const uint32_t do_base = smem_u32(smem + L::DO_OFF + s * L::TILE);
-        if (PIPELINED) {
-          if (t + 1 < n_it) issue_scores(t + 1);   // runs on the tensor core while the compute warps work on block t
-        } else {
-          // when dQ aliases S (D = 128) the previous dQ partial must be drained first
-          if (t > 0) mbar_wait(dq_empty, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
-          issue_scores(t);
+        const int s = t & 1, q = (i0 + t) * 128 + lane * 4;
+        float* ld = reinterpret_cast<float*>(smem + L::LD_OFF) + s * 256;
+        const size_t at = ((size_t)b * p.H + h) * p.S + q;
+        float lv[4], dv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {   // queries beyond S: exp2(s - inf) = 0
+          lv[j] = q + j < p.S ? p.LSE[at + j] * -1.4426950408889634f : -INFINITY;
+          dv[j] = q + j < p.S ? p.delta[at + j] * -p.scale : 0.f;
         }
-        // P and dS are in shared memory once the compute warps arrive here
-        mbar_wait(ds_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_MISC);
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_ss(tmem_base + TM_DV, desc_at(make_smem_desc_sw128(p_base, 16384, 1024), kk * 2048),
-                  desc_at(make_smem_desc_sw128(do_base, 16384, 1024), kk * 2048), idesc_dkv, (t | kk) ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_ss(tmem_base + TM_DK, desc_at(make_smem_desc_sw128(ds_base, 16384, 1024), kk * 2048),
-                  desc_at(make_smem_desc_sw128(q_base, 16384, 1024), kk * 2048), idesc_dkv, (t | kk) ? 1u : 0u);
-        if (D == 64 && t > 0) mbar_wait(dq_empty, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_ss(tmem_base + TM_DQ,
-                  desc_at(make_smem_desc_sw128(ds_base, 16, 1024), (kk >> 2) * 16384 + (kk & 3) * 32),
-                  desc_at(make_smem_desc_sw128(k_base, 16384, 1024), kk * 2048), idesc_dq, kk ? 1u : 0u);
-        umma_commit(dq_full);
-        umma_commit(pds_empty);
-        umma_commit(&q_empty[s]);
-        umma_commit(&do_empty[s]);
+        mbar_wait(&ld_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY);
+        *reinterpret_cast<float4*>(ld + lane * 4) = make_float4(lv[0], lv[1], lv[2], lv[3]);
+        *reinterpret_cast<float4*>(ld + 128 + lane * 4) = make_float4(dv[0], dv[1], dv[2], dv[3]);
+        mbar_arrive(&ld_full[s]);
       }
-      umma_commit(dkv_full);
+    } else if (warp == 12) {
+      // -------------------------------------------------------------- MMA issuer
+      if (elect_one()) {
+        constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
+        constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, 0, 1);   // dV, dK: A K-major (TMEM / smem), B MN-major
+        constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, 1, 1);
+        const uint32_t k_base = smem_u32(smem + L::K_OFF), v_base = smem_u32(smem + L::V_OFF);
+        const uint32_t q_base = smem_u32(smem + L::Q_OFF), do_base = smem_u32(smem + L::DO_OFF);
+        const uint32_t ds_base = smem_u32(smem + L::DS_OFF);
+        const uint64_t k_kd = make_smem_desc_sw128(k_base, 16, 1024), k_mn = make_smem_desc_sw128(k_base, 16384, 1024);
+        const uint64_t v_kd = make_smem_desc_sw128(v_base, 16, 1024);
+        const uint64_t q_kd = make_smem_desc_sw128(q_base, 16, 1024), q_mn = make_smem_desc_sw128(q_base, 16384, 1024);
+        const uint64_t do_kd = make_smem_desc_sw128(do_base, 16, 1024), do_mn = make_smem_desc_sw128(do_base, 16384, 1024);
+        const uint64_t ds_kd = make_smem_desc_sw128(ds_base, 16, 1024), ds_mn = make_smem_desc_sw128(ds_base, 16384, 1024);
+        auto issue_s = [&](int t) {   // S^T = K Q_t^T
+          const uint32_t so = (t & 1) * L::TILE;
+          mbar_wait(&q_full[t & 1], (t >> 1) & 1, abort_flag, p.status, TB_ERR_WAIT_FULL);
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < KCH; ++c)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_ss(tmem_base + TM_S, desc_at(k_kd, c * 16384 + k * 32), desc_at(q_kd, so + c * 16384 + k * 32), idesc_s,
+                      (c | k) ? 1u : 0u);
+          umma_commit(s_full);
+        };
+        auto issue_dp = [&](int t) {  // dP^T = V dO_t^T; its columns were read before ds_full[t - 1]
+          const uint32_t sdo = (t % DOST) * L::TILE;
+          mbar_wait(&do_full[t % DOST], (t / DOST) & 1, abort_flag, p.status, TB_ERR_WAIT_FULL);
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < KCH; ++c)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_ss(tmem_base + TM_DP, desc_at(v_kd, c * 16384 + k * 32), desc_at(do_kd, sdo + c * 16384 + k * 32), idesc_s,
+                      (c | k) ? 1u : 0u);
+          umma_commit(dp_full);
+        };
+        mbar_wait(kv_full, 0, abort_flag, p.status, TB_ERR_WAIT_FULL);
+        issue_s(0);
+        issue_dp(0);
+        for (int t = 0; t < n_it; ++t) {
+          const uint32_t so = (t & 1) * L::TILE, sdo = (t % DOST) * L::TILE;
+          mbar_wait(p_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_MISC);
+          if (ROOMY && t + 1 < n_it) issue_s(t + 1);   // S^T[t] has been read
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)   // dV += P^T dO_t
+            umma_ts(tmem_base + TM_DV, tmem_base + TM_P + (kk >> 2) * P_HALF + (kk & 3) * 8, desc_at(do_mn, sdo + kk * 2048), idesc_kv,
+                    (t | kk) ? 1u : 0u);
+          umma_commit(dv_done);
+          umma_commit(&do_empty[t % DOST]);
+          if (!ROOMY && t + 1 < n_it) {
+            mbar_wait(dv_done, t & 1, abort_flag, p.status, TB_ERR_WAIT_MISC);  // P^T[t] is no longer read
+            issue_s(t + 1);
+          }
+          mbar_wait(ds_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_MISC);
+          if (ROOMY && t + 1 < n_it) issue_dp(t + 1);
+          if (ROOMY && t > 0) mbar_wait(dq_empty, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)   // dQ before dK: its way out is the longer one
+            umma_ss(tmem_base + TM_DQ, desc_at(ds_mn, kk * 2048), desc_at(k_mn, kk * 2048), idesc_dq, kk ? 1u : 0u);
+          umma_commit(dq_full);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_ss(tmem_base + TM_DK, desc_at(ds_kd, (kk >> 2) * 16384 + (kk & 3) * 32), desc_at(q_mn, so + kk * 2048), idesc_kv,
+                    (t | kk) ? 1u : 0u);
+          umma_commit(ds_empty);
+          umma_commit(&q_empty[t & 1]);
+          if (!ROOMY && t + 1 < n_it) {
+            mbar_wait(dq_empty, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);
+            issue_dp(t + 1);
+          }
+        }
+        umma_commit(dkv_full);
+      }
     }
-  } else {
-    // ---------------------------------------------------------------- compute (8 warps)
-    // Two warps per group of 32 rows: warps 0-3 take key columns 0-63 (and the first half of the
-    // dQ / dK / dV columns), warps 4-7 the rest; no exchange is needed, L and delta are per row.
-    const int half = warp >> 2;
-    const int row = (warp & 3) * 32 + lane;
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const float sl2 = p.scale * 1.4426950408889634f;
-    uint8_t* p_smem = smem + L::P_OFF;
-    uint8_t* ds_smem = smem + L::DS_OFF;
-    const int sw = row & 7;
-    // dQ partial of query block tt: TMEM -> this warp's staging rows -> one 4 KB bulk reduce-add per 32 columns. The
-    // accumulator keeps the staged order (the cast pass undoes it), so that a warp's rows are one contiguous run: as
-    // 16-byte reductions of every lane into its own row they reached 1.1 to 1.5 TB/s of L2 and bounded the kernel.
-    uint8_t* dq_stage = smem + L::DQ_OFF + warp * 4096;
-    auto drain_dq = [&](int tt) {
-      mbar_wait(dq_full, tt & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
+  } else if (warp >= 8) {
+    // ---------------------------------------------------------------- dQ out (4 warps, one TMEM lane quarter each)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    // A warp's rows leave as one 4 KB bulk reduce-add per 32 columns; the accumulator keeps the staged order (the cast
+    // pass undoes it). As 16-byte reductions of every lane into its own row they reached 1.1 to 1.5 TB/s of L2.
+    uint8_t* stage = smem + L::DQ_OFF + (warp & 3) * 8192;
+    const int sw = lane & 7;
+    for (int t = 0; t < n_it; ++t) {
+      mbar_wait(dq_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
-      float* dq_blk = p.dQ_acc + (((size_t)bh * n_blk + i0 + tt) * (D / 32)) * 4096 + (warp & 3) * 1024;
-#pragma unroll 1
-      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + TM_DQ + c * 32 + lane_off, v);
+      float* dq_blk = p.dQ_acc + (((size_t)bh * n_blk + i0 + t) * (D / 32)) * 4096 + (warp & 3) * 1024;
+#pragma unroll
+      for (int c = 0; c < D / 32; c += 2) {
+        // both columns groups to registers first: with the last pair the columns are free before anything is staged
+        uint32_t v[2][32];
+        tmem_ld32(tmem_base + TM_DQ + c * 32 + lane_off, v[0]);
+        tmem_ld32(tmem_base + TM_DQ + c * 32 + 32 + lane_off, v[1]);
         tmem_wait_ld();
-        if (lane == 0) bulk_wait_read_all();  // the previous run has left the staging rows
+        if (c == D / 32 - 2) {
+          tc_fence_before();
+          mbar_arrive(dq_empty);
+        }
+        if (lane == 0) bulk_wait_read_all();  // the previous pair has left the staging rows
         __syncwarp();
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<uint4*>(dq_stage + lane * 128 + ((g ^ sw) << 4)) =
-              make_uint4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(stage + k * 4096 + lane * 128 + ((g ^ sw) << 4)) =
+                make_uint4(v[k][g * 4], v[k][g * 4 + 1], v[k][g * 4 + 2], v[k][g * 4 + 3]);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_blk + c * 4096),
-                       "r"(smem_u32(dq_stage)), "r"(4096)
-                       : "memory");
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_blk + (c + k) * 4096),
+                         "r"(smem_u32(stage + k * 4096)), "r"(4096)
+                         : "memory");
           bulk_commit();
         }
       }
-      tc_fence_before();
-      mbar_arrive(dq_empty);
-    };
+    }
+    if (lane == 0) bulk_wait_all();
+  } else {
+    // ---------------------------------------------------------------- compute (8 warps)
+    // Two warps per group of 32 key rows: warps 0-3 take queries 0-63 of every block (and the first half of the dK / dV
+    // columns at the end), warps 4-7 the rest; no exchange is needed, L and delta are per query.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+    const int half = warp >> 2;
+    const int row = (warp & 3) * 32 + lane;
+    const int key = kv0 + row;
+    const float sl2 = p.scale * 1.4426950408889634f;
+    uint8_t* ds_row = smem + L::DS_OFF + half * 16384 + row * 128;
+    const int sw = row & 7;
+    const uint32_t tp = tmem_base + TM_P + half * P_HALF + lane_off;
+    const uint32_t ts = tmem_base + TM_S + half * 64 + lane_off, tdp = tmem_base + TM_DP + half * 64 + lane_off;
     for (int t = 0; t < n_it; ++t) {
-      const int qi = (i0 + t) * 128 + row;
-      const bool q_ok = qi < p.S;
-      const size_t stat_idx = ((size_t)b * p.H + h) * p.S + (q_ok ? qi : 0);
-      const float Lr = q_ok ? p.LSE[stat_idx] * 1.4426950408889634f : INFINITY;
-      const float dr = q_ok ? p.delta[stat_idx] : 0.f;
-      const bool need_mask = (p.causal && (i0 + t) == jb) || (kv0 + 128 > p.S);
-      const int col_limit = p.causal ? min(qi, p.S - 1) : p.S - 1;
+      const float* ld = reinterpret_cast<const float*>(smem + L::LD_OFF) + (t & 1) * 256 + half * 64;
+      const bool need_mask = (p.causal && t == 0) || kv0 + 128 > p.S;   // with a causal mask block 0 is the diagonal one
+      // first query (relative to this half) that sees the key: none for a key beyond S
+      const int first = key >= p.S ? 1 << 30 : p.causal ? key - ((i0 + t) * 128 + half * 64) : 0;
+      float e0[32], e1[32];
+      uint32_t v0[32], v1[32], pk[16];
+      mbar_wait(&ld_full[t & 1], (t >> 1) & 1, abort_flag, p.status, TB_ERR_WAIT_FULL);
       mbar_wait(s_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
-      // this thread's 64 score columns go to registers at once, so that the tensor core may overwrite S
-      uint32_t sv0[32], sv1[32];
-      tmem_ld32(tmem_base + TM_S + (half * 2) * 32 + lane_off, sv0);
-      tmem_ld32(tmem_base + TM_S + (half * 2 + 1) * 32 + lane_off, sv1);
+      // all 64 scores at once: the load's latency is paid once, and P^T may land on the same half's columns
+      tmem_ld32(ts, v0);
+      tmem_ld32(ts + 32, v1);
       tmem_wait_ld();
-      if (PIPELINED) {
-        tc_fence_before();
-        mbar_arrive(s_free);
-      }
+      if (need_mask) fa_bwd_p<true>(v0, ld, sl2, first, e0, pk);
+      else fa_bwd_p<false>(v0, ld, sl2, first, e0, pk);
+      if (ROOMY && t > 0) mbar_wait(dv_done, (t - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);  // P^T[t - 1] is read
+      tmem_st16(tp, pk);
+      if (need_mask) fa_bwd_p<true>(v1, ld + 32, sl2, first - 32, e1, pk);
+      else fa_bwd_p<false>(v1, ld + 32, sl2, first - 32, e1, pk);
+      tmem_st16(tp + 16, pk);
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(p_full);
       mbar_wait(dp_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
-      // the previous iteration's MMAs must be done reading P / dS from shared memory
-      mbar_wait(pds_empty, (t & 1) ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY);
       tc_fence_after();
+      tmem_ld32(tdp, v0);
+      tmem_ld32(tdp + 32, v1);
+      tmem_wait_ld();
+      mbar_wait(ds_empty, (t & 1) ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY);  // dK / dQ of block t - 1 have read dS^T
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = half * 2 + cc;
-        uint32_t dv[32];
-        tmem_ld32(tmem_base + TM_DP + c * 32 + lane_off, dv);
-        tmem_wait_ld();
-        if (PIPELINED && cc == 1) {
-          tc_fence_before();
-          mbar_arrive(dp_free);
-        }
-        uint32_t pp[16], dd[16];
-        const uint32_t (&sv)[32] = cc == 0 ? sv0 : sv1;
-        if (need_mask) fa_bwd_p_ds<true>(sv, dv, sl2, Lr, p.scale, dr, kv0 + c * 32, col_limit, pp, dd);
-        else fa_bwd_p_ds<false>(sv, dv, sl2, Lr, p.scale, dr, kv0 + c * 32, col_limit, pp, dd);
-        // columns c*32 .. c*32+31 = four 16-byte chunks of sub-tile c/2 (64 keys per sub-tile)
-        const int sub = c >> 1;
+      for (int c = 0; c < 2; ++c) {
+        fa_bwd_ds(c == 0 ? v0 : v1, ld + 128 + c * 32, p.scale, c == 0 ? e0 : e1, pk);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int ch = (c & 1) * 4 + g;
-          const int off = sub * 16384 + row * 128 + ((ch ^ sw) << 4);
-          *reinterpret_cast<uint4*>(p_smem + off) = make_uint4(pp[g * 4], pp[g * 4 + 1], pp[g * 4 + 2], pp[g * 4 + 3]);
-          *reinterpret_cast<uint4*>(ds_smem + off) = make_uint4(dd[g * 4], dd[g * 4 + 1], dd[g * 4 + 2], dd[g * 4 + 3]);
-        }
+        for (int g = 0; g < 4; ++g)
+          *reinterpret_cast<uint4*>(ds_row + (((c * 4 + g) ^ sw) << 4)) = make_uint4(pk[g * 4], pk[g * 4 + 1], pk[g * 4 + 2], pk[g * 4 + 3]);
       }
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(ds_full);
-      if (PIPELINED) {
-        if (t > 0) drain_dq(t - 1);   // finished long ago: the MMAs of block t - 1 ran under this block's exponentials
-      } else {
-        drain_dq(t);
-      }
+      mbar_arrive(&ld_empty[t & 1]);
     }
-    if (PIPELINED && n_it > 0) drain_dq(n_it - 1);
-    if (lane == 0) bulk_wait_all();
     // dK, dV of this key block: thread = key row
     mbar_wait(dkv_full, 0, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
     tc_fence_after();
-    const int kvi = kv0 + row;
-    const bool kv_ok = kvi < p.S;
-    __nv_bfloat16* dk_row = p.dK + ((size_t)b * p.S + (kv_ok ? kvi : 0)) * p.dkv_stride + (size_t)h * D;
-    __nv_bfloat16* dv_row = p.dV + ((size_t)b * p.S + (kv_ok ? kvi : 0)) * p.dkv_stride + (size_t)h * D;
+    const bool kv_ok = key < p.S;
+    __nv_bfloat16* dk_row = p.dK + ((size_t)b * p.S + (kv_ok ? key : 0)) * p.dkv_stride + (size_t)h * D;
+    __nv_bfloat16* dv_row = p.dV + ((size_t)b * p.S + (kv_ok ? key : 0)) * p.dkv_stride + (size_t)h * D;
 #pragma unroll 1
     for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
       uint32_t kvv[32], vvv[32];
@@ -396,7 +449,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == 12) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
