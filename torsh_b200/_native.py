@@ -16,6 +16,7 @@ import torch
 _LIBDIR = Path(__file__).resolve().parent / "lib"
 _lock = threading.Lock()
 _cuda_lib = None
+_cuda_present = False
 _host_lib = None
 _status = {}
 launch_count = 0  # kernels of this library launched so far (incremented by the op wrappers)
@@ -73,9 +74,20 @@ def cuda_available() -> bool:
 
 
 def require_cuda():
+    # once the library is loaded on a machine that has a GPU there is nothing left to ask (is_available() reads the
+    # environment on every call, which cost a launch about 3 us)
+    if _cuda_present:
+        return _cuda_lib
+    return _find_cuda()
+
+
+def _find_cuda():
+    global _cuda_present
     if not torch.cuda.is_available():
         raise NativeError("this op needs a CUDA device")
-    return cuda()
+    lib = cuda()
+    _cuda_present = True
+    return lib
 
 
 def check(rc: int, what: str = "") -> None:
@@ -96,8 +108,8 @@ def stream_ptr(stream: torch.cuda.Stream | None = None) -> c_void_p:
     if d != _bound_device:
         cuda().tb_set_device(d)
         _bound_device = d
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return c_void_p(s.cuda_stream)
+    # the handle itself: building a torch.cuda.Stream to read it from cost a launch about 7 us
+    return c_void_p(torch._C._cuda_getCurrentRawStream(d) if stream is None else stream.cuda_stream)
 
 
 def ptr(t: torch.Tensor | None) -> c_void_p:
@@ -116,6 +128,12 @@ def status_word(device: torch.device | int | None = None) -> torch.Tensor:
         if RuntimeConfig.global_().kernel_checks:
             enable_kernel_checks(True, key)
     return st
+
+
+def status_ptr(device: torch.device) -> int:
+    """Address of :func:`status_word` of a CUDA tensor's device (the words live as long as the process)."""
+    st = _status.get(device.index)
+    return (st if st is not None else status_word(device)).data_ptr()
 
 
 def enable_kernel_checks(on: bool = True, device: int | None = None) -> None:

@@ -8,7 +8,8 @@ import torch
 from .. import _native as nv
 
 P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float
-_sigs_done: set[str] = set()
+_fns: dict = {}
+_KERNEL_DTYPES = (torch.bfloat16, torch.float32)
 
 
 def dtype_code(t: torch.Tensor) -> int:
@@ -21,7 +22,10 @@ def dtype_code(t: torch.Tensor) -> int:
 
 def kernel_ok(*tensors: torch.Tensor) -> bool:
     """True when every tensor is a CUDA bf16/fp32 tensor (the kernels' domain)."""
-    return all(t is None or (t.is_cuda and t.dtype in (torch.bfloat16, torch.float32)) for t in tensors)
+    for t in tensors:
+        if t is not None and not (t.is_cuda and t.dtype in _KERNEL_DTYPES):
+            return False
+    return True
 
 
 def aligned(t: torch.Tensor) -> torch.Tensor:
@@ -35,12 +39,12 @@ def aligned(t: torch.Tensor) -> torch.Tensor:
 
 def fn(name: str, argtypes):
     """Fetch a launcher from the CUDA library and set its signature once."""
-    lib = nv.require_cuda()
-    f = getattr(lib, name)
-    if name not in _sigs_done:
+    f = _fns.get(name)
+    if f is None:
+        f = getattr(nv.require_cuda(), name)
         f.restype = ctypes.c_int
         f.argtypes = argtypes
-        _sigs_done.add(name)
+        _fns[name] = f
     return f
 
 
@@ -48,5 +52,7 @@ _KERNELS_PER_CALL = {"tb_flash_attn_bwd": 3, "tb_lamb_multi": 2, "tb_bn_fwd": 3,
 
 
 def call(name: str, argtypes, *args):
-    nv.check(fn(name, argtypes)(*args), name)
+    rc = fn(name, argtypes)(*args)
+    if rc != 0:
+        nv.check(rc, name)
     nv.launch_count += _KERNELS_PER_CALL.get(name, 1)

@@ -19,7 +19,7 @@ _BWD = [P] * 11 + [I, I, I, I, L, L, L, L, L, F, I, P, P]
 
 def _fwd(q, k, v, out, lse, B, S, H, D, q_stride, kv_stride, scale, causal):
     call("tb_flash_attn_fwd", _FWD, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S,
-         H, D, q_stride, kv_stride, out.stride(0), float(scale), int(causal), nv.status_word(q.device).data_ptr(),
+         H, D, q_stride, kv_stride, out.stride(0), float(scale), int(causal), nv.status_ptr(q.device),
          nv.stream_ptr())
 
 
@@ -29,7 +29,7 @@ def _bwd(q, k, v, o, do, lse, dq, dk, dv, B, S, H, D, q_stride, kv_stride, dqkv_
     call("tb_flash_attn_bwd", _BWD, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(),
          lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), B, S, H, D,
          q_stride, kv_stride, o.stride(0), do.stride(0), dqkv_stride, float(scale), int(causal),
-         nv.status_word(q.device).data_ptr(), nv.stream_ptr())
+         nv.status_ptr(q.device), nv.stream_ptr())
 
 
 class _FlashQKVPacked(torch.autograd.Function):

@@ -51,9 +51,8 @@ def _conv3x3_gemm(x, wm, cout, mode):
     """Implicit-GEMM 3x3/1/1 convolution (mode 1) or its input gradient (mode 2): no column matrix is written."""
     n, h, w, c = x.shape
     y = torch.empty(n * h * w, cout, dtype=torch.bfloat16, device=x.device)
-    st = nv.status_word(x.device)
     call("tb_conv3x3_gemm", [P, P, P, I, I, I, I, I, I, I, I, I, P, P], x.data_ptr(), wm.data_ptr(), y.data_ptr(), n, h, w, c,
-         cout, mode, wm.stride(0), cout, 0, st.data_ptr(), nv.stream_ptr())
+         cout, mode, wm.stride(0), cout, 0, nv.status_ptr(x.device), nv.stream_ptr())
     return y
 
 
@@ -111,9 +110,8 @@ class _Conv2dFn(torch.autograd.Function):
                     tiles = ((co + 127) // 128) * ((kpad + 255) // 256)
                     sk = max(1, min(296 // max(tiles, 1), kb // 16))
                     g = torch.zeros(co, kpad, dtype=torch.float32, device=dy.device)
-                    st = nv.status_word(dy.device)
                     call("tb_conv3x3_wgrad", [P, P, P, I, I, I, I, I, I, I, I, P, P], dy2.data_ptr(), a.data_ptr(), g.data_ptr(),
-                         n, h, w, c, co, kpad, sk, 0, st.data_ptr(), nv.stream_ptr())
+                         n, h, w, c, co, kpad, sk, 0, nv.status_ptr(dy.device), nv.stream_ptr())
                     dw = g[:, :k].reshape(co, kh, kw, c).permute(0, 3, 1, 2).to(ctx.wdtype)
                     return dx, dw, None, None
                 a = _im2col(a, kh, kw, stride, pad, kpad)

@@ -9,6 +9,7 @@ pass. Kernel: ``csrc/kernels/gemm_sm100.cu``. The reference's matmul is a 2-D na
 from __future__ import annotations
 
 import ctypes
+import os
 
 import torch
 
@@ -40,14 +41,12 @@ def gemm_autotune(on: bool = True, path: str | None = None):
     if not on:
         _autotune = None
         return None
-    import os
     from ..core.backend import Autotuner
     _autotune = Autotuner(path or os.environ.get("TORSH_GEMM_TUNE_FILE"), warmup=1, iters=3)
     return _autotune
 
 
 def _env_autotune():
-    import os
     if _autotune is None and os.environ.get("TORSH_GEMM_AUTOTUNE", "0") == "1":
         gemm_autotune(True)
     return _autotune
@@ -133,7 +132,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
         raster_m = N > 4 * M or (N >= 16384 and N > M)
     if raster_m:
         flags |= EPI_RASTER_M
-    st = nv.status_word(a.device)
+    st = nv.status_ptr(a.device)
     # FSDP full shard: the first GEMM that reads a weight of a unit whose un-shard is pending performs that un-shard
     # itself (copy CTAs of the same launch pull the shards while the tiles are computed)
     unit = getattr(b, "_tb_fsdp_unit", None)
@@ -143,14 +142,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
             rc = _lib().tb_fsdp_ag_gemm(
                 a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a_major, b_major, a.stride(0), b.stride(0),
                 out.stride(0), nv.ptr(bias), nv.ptr(residual), residual.stride(0) if residual is not None else 0,
-                nv.ptr(preact_out), nv.ptr(dgelu_aux), flags, bn, *g, st.data_ptr(), nv.stream_ptr())
+                nv.ptr(preact_out), nv.ptr(dgelu_aux), flags, bn, *g, st, nv.stream_ptr())
             nv.check(rc, "tb_fsdp_ag_gemm")
             nv.launch_count += 2
             return out
     rc = _lib().tb_gemm_bf16(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a_major, b_major, a.stride(0), b.stride(0),
         out.stride(0), nv.ptr(bias), nv.ptr(residual), residual.stride(0) if residual is not None else 0,
-        nv.ptr(preact_out), nv.ptr(dgelu_aux), flags, split_k, bn, st.data_ptr(), nv.stream_ptr())
-    nv.check(rc, "tb_gemm_bf16")
+        nv.ptr(preact_out), nv.ptr(dgelu_aux), flags, split_k, bn, st, nv.stream_ptr())
+    if rc != 0:
+        nv.check(rc, "tb_gemm_bf16")
     nv.launch_count += 1
     return out
