@@ -210,7 +210,7 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Warp-per-row forms for rows of at most 32 * VPL 16-byte vectors (H <= 2048 bf16, 1024 fp32). A warp owns a row: its
+// Warp-per-row form of the forward for rows of at most 32 * VPL 16-byte vectors (H <= 2048 bf16, 1024 fp32). A warp owns a row: its
 // statistics are two shuffle reductions with no block barrier, eight rows are in flight per CTA and the next row of
 // every warp is requested before the current one is reduced. With one CTA per row a 2 KB row left too few bytes in
 // flight per SM and two block barriers per row on the critical path (0.43 of the copy bandwidth at 32768 x 1024).
@@ -299,101 +299,177 @@ __global__ void __launch_bounds__(NORM_WARPS * 32, VPL <= 4 ? 2 : 1) norm_fwd_wa
   }
 }
 
-// Same arithmetic as norm_bwd_kernel. Every lane keeps fp32 partial sums of d(gamma) / d(beta) for its own columns
-// over all rows of its warp; the CTA's eight warps then add theirs in shared memory (2 * H floats) and the CTA writes
-// one partial row of the workspace (or adds into the gradients with atomics when there is none).
-template <typename T, int VPL, bool RMS>
-__global__ void __launch_bounds__(NORM_WARPS * 32) norm_bwd_warp_kernel(
+// Backward for rows of up to 8192 elements: same arithmetic as norm_bwd_kernel. A team of G warps owns a row (16 elements a
+// lane, 8 where that leaves fewer lanes idle) and walks rows with the next two or three already on their way: every lane
+// copies its own vectors of x, dy and dres into a ring in shared memory (cp.async without a barrier: a lane reads only what it
+// copied), and the statistics travel one row ahead. With the next row in registers there was room for 8 warps at 255
+// registers, and every row began with a load of its mean: 82 us at 32768 x 1024 bf16, where this form takes 48 (31 at the copy
+// rate); 8192 x 1024 with a residual gradient 32.5 -> 18.2, 1999 x 4096 fp32 29.3 -> 18.2, 20000 x 1600 89.6 -> 59.6. d(gamma) / d(beta) partial
+// sums stay in registers for all rows of a team, meet in shared memory once and leave as one partial row per CTA.
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+
+template <typename T, int VPL, int NW, bool RMS>
+__global__ void __launch_bounds__(NW * 32, 1) norm_bwd_ring_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma, const float* __restrict__ mean_in,
     const float* __restrict__ rstd_in, const T* __restrict__ dres, T* __restrict__ dx, float* __restrict__ dgamma,
-    float* __restrict__ dbeta, float* __restrict__ partial, int rows, int H) {
+    float* __restrict__ dbeta, float* __restrict__ partial, int rows, int H, int G) {
   constexpr int N = Vec16<T>::N;
-  extern __shared__ float nb_sums[];  // [2][H]
+  extern __shared__ __align__(16) uint8_t nb_smem[];
+  __shared__ float2 exch[2][NW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nvec = H / N;
-  const int nwarps = gridDim.x * NORM_WARPS;
-  float gf[VPL][N], dg[VPL][N], db[VPL][N];
+  const int teams = NW / G, team = warp / G, member = warp - team * G;
+  const int nvec = H / N, narr = dres ? 3 : 2, stages = dres ? 2 : 3;
+  const bool active = team < teams;
+  const int step = gridDim.x * teams;
+  float2 dg[VPL][N / 2], db[VPL][N / 2];
+  Vec16<T> gv[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
+    const int v = member * 32 + lane + i * 32 * G;
 #pragma unroll
-    for (int j = 0; j < N; ++j) dg[i][j] = db[i][j] = gf[i][j] = 0.f;
-    if (lane + 32 * i < nvec) {
-      Vec16<T> t;
-      t.load_nc(gamma + (lane + 32 * i) * N);
-      t.get(gf[i]);
-    }
+    for (int j = 0; j < N / 2; ++j) dg[i][j] = db[i][j] = make_float2(0.f, 0.f);
+    if (active && v < nvec) gv[i].load_nc(gamma + v * N);
+    else gv[i].raw = make_uint4(0, 0, 0, 0);
   }
-  Vec16<T> nx[VPL], nd[VPL], nr[VPL];
-  auto request = [&](int r) {
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int v = lane + 32 * i;
-      if (v < nvec) {
-        nx[i].load(x + (size_t)r * H + v * N);
-        nd[i].load(dy + (size_t)r * H + v * N);
-        if (dres) nr[i].load(dres + (size_t)r * H + v * N);
-      }
-    }
+  auto slot = [&](int stage, int arr, int i) {
+    return nb_smem + ((((size_t)stage * NW + warp) * narr + arr) * VPL + i) * 512 + lane * 16;
   };
-  int row = blockIdx.x * NORM_WARPS + warp;
-  if (row < rows) request(row);
-  const float inv_h = 1.f / (float)H;
-  for (; row < rows; row += nwarps) {
-    const float mean = RMS ? 0.f : mean_in[row];
-    const float rstd = rstd_in[row];
-    float xh[VPL][N], dyg[VPL][N], res[VPL][N];
-    float s1 = 0.f, s2 = 0.f;
+  auto request = [&](int row, int stage) {
+    if (row < rows) {
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      if (lane + 32 * i < nvec) {
-        float xf[N], df[N];
-        nx[i].get(xf);
-        nd[i].get(df);
-        if (dres) nr[i].get(res[i]);
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-          xh[i][j] = (xf[j] - mean) * rstd;
-          dyg[i][j] = df[j] * gf[i][j];
-          dg[i][j] += df[j] * xh[i][j];
-          db[i][j] += df[j];
-          s1 += dyg[i][j];
-          s2 += dyg[i][j] * xh[i][j];
+      for (int i = 0; i < VPL; ++i) {
+        const int v = member * 32 + lane + i * 32 * G;
+        if (v < nvec) {
+          const size_t at = (size_t)row * H + v * N;
+          cp_async16(slot(stage, 0, i), x + at);
+          cp_async16(slot(stage, 1, i), dy + at);
+          if (dres) cp_async16(slot(stage, 2, i), dres + at);
         }
       }
     }
-    if (row + nwarps < rows) request(row + nwarps);
-    s1 = RMS ? 0.f : warp_sum(s1) * inv_h;
-    s2 = warp_sum(s2) * inv_h;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int v = lane + 32 * i;
-      if (v < nvec) {
-        float o[N];
-#pragma unroll
-        for (int j = 0; j < N; ++j) o[j] = (dres ? res[i][j] : 0.f) + rstd * (dyg[i][j] - s1 - xh[i][j] * s2);
-        Vec16<T> t;
-        t.set(o);
-        t.store(dx + (size_t)row * H + v * N);
-      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const float inv_h = 1.f / (float)H;
+  if (active) {
+    int row = blockIdx.x * teams + team;
+    for (int k = 0; k < stages; ++k) request(row + k * step, k);
+    int stage = 0, par = 0;
+    // the next row's statistics travel one row ahead, too: read when needed they put a memory latency into every row
+    float mean_next = 0.f, rstd_next = 0.f;
+    if (row < rows) {
+      if (!RMS) mean_next = mean_in[row];
+      rstd_next = rstd_in[row];
     }
-  }
-  // the eight warps take turns adding their column sums into shared memory
-  for (int w = 0; w < NORM_WARPS; ++w) {
-    if (warp == w) {
+    for (; row < rows; row += step) {
+      const float mean = mean_next, rstd = rstd_next;
+      if (row + step < rows) {
+        if (!RMS) mean_next = mean_in[row + step];
+        rstd_next = rstd_in[row + step];
+      }
+      if (dres) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 2;" ::: "memory");
+      // packed two-wide fp32 arithmetic: the row's instructions, not its bytes, were the larger share
+      const float2 nm2 = make_float2(-mean, -mean), r2 = make_float2(rstd, rstd);
+      float2 s1v = make_float2(0.f, 0.f), s2v = make_float2(0.f, 0.f);
+      Vec16<T> xv[VPL], dv[VPL];
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
-        const int v = lane + 32 * i;
+        if (member * 32 + lane + i * 32 * G < nvec) {
+          xv[i].raw = *reinterpret_cast<const uint4*>(slot(stage, 0, i));
+          dv[i].raw = *reinterpret_cast<const uint4*>(slot(stage, 1, i));
+          float xf[N], df[N], gf[N];
+          xv[i].get(xf);
+          dv[i].get(df);
+          gv[i].get(gf);
+#pragma unroll
+          for (int j = 0; j < N; j += 2) {
+            const float2 d2 = make_float2(df[j], df[j + 1]);
+            const float2 xh = __fmul2_rn(__fadd2_rn(make_float2(xf[j], xf[j + 1]), nm2), r2);
+            const float2 dyg = __fmul2_rn(d2, make_float2(gf[j], gf[j + 1]));
+            dg[i][j / 2] = __ffma2_rn(d2, xh, dg[i][j / 2]);
+            if (!RMS) {
+              db[i][j / 2] = __fadd2_rn(db[i][j / 2], d2);
+              s1v = __fadd2_rn(s1v, dyg);
+            }
+            s2v = __ffma2_rn(dyg, xh, s2v);
+          }
+        }
+      }
+      float s1 = s1v.x + s1v.y, s2 = s2v.x + s2v.y;
+      s1 = RMS ? 0.f : warp_sum(s1);
+      s2 = warp_sum(s2);
+      if (G > 1) {  // the team's warps add their sums in the same order (two buffers: the next row may be ahead)
+        if (lane == 0) exch[par][warp] = make_float2(s1, s2);
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(G * 32) : "memory");
+        s1 = s2 = 0.f;
+        for (int m = 0; m < G; ++m) {
+          const float2 e = exch[par][team * G + m];
+          s1 += e.x;
+          s2 += e.y;
+        }
+        par ^= 1;
+      }
+      const float2 ns1 = make_float2(-s1 * inv_h, -s1 * inv_h), ns2 = make_float2(-s2 * inv_h, -s2 * inv_h);
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        const int v = member * 32 + lane + i * 32 * G;
+        if (v < nvec) {
+          float xf[N], df[N], gf[N], o[N];
+          xv[i].get(xf);
+          dv[i].get(df);
+          gv[i].get(gf);
+          if (dres) {
+            Vec16<T> r;
+            r.raw = *reinterpret_cast<const uint4*>(slot(stage, 2, i));
+            r.get(o);
+          } else {
+#pragma unroll
+            for (int j = 0; j < N; ++j) o[j] = 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < N; j += 2) {
+            const float2 xh = __fmul2_rn(__fadd2_rn(make_float2(xf[j], xf[j + 1]), nm2), r2);
+            float2 t2 = __ffma2_rn(make_float2(df[j], df[j + 1]), make_float2(gf[j], gf[j + 1]), ns1);
+            t2 = __ffma2_rn(xh, ns2, t2);
+            t2 = __ffma2_rn(t2, r2, make_float2(o[j], o[j + 1]));
+            o[j] = t2.x;
+            o[j + 1] = t2.y;
+          }
+          Vec16<T> t;
+          t.set(o);
+          t.store(dx + (size_t)row * H + v * N);
+        }
+      }
+      request(row + stages * step, stage);
+      if (++stage == stages) stage = 0;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // the teams take turns adding their column sums into [2][H] floats over the ring's memory
+  float* sums = reinterpret_cast<float*>(nb_smem);
+  for (int t = 0; t < teams; ++t) {
+    if (active && team == t) {
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        const int v = member * 32 + lane + i * 32 * G;
         if (v < nvec) {
 #pragma unroll
-          for (int j = 0; j < N; ++j) {
-            float* pg = nb_sums + v * N + j;
-            if (w == 0) {
-              pg[0] = dg[i][j];
-              pg[H] = db[i][j];
-            } else {
-              pg[0] += dg[i][j];
-              pg[H] += db[i][j];
+          for (int j = 0; j < N; j += 4) {
+            float4* pg = reinterpret_cast<float4*>(sums + v * N + j);
+            float4* pb = reinterpret_cast<float4*>(sums + H + v * N + j);
+            float4 a = make_float4(dg[i][j / 2].x, dg[i][j / 2].y, dg[i][j / 2 + 1].x, dg[i][j / 2 + 1].y);
+            float4 c = make_float4(db[i][j / 2].x, db[i][j / 2].y, db[i][j / 2 + 1].x, db[i][j / 2 + 1].y);
+            if (t > 0) {
+              const float4 a0 = *pg, c0 = *pb;
+              a.x += a0.x; a.y += a0.y; a.z += a0.z; a.w += a0.w;
+              c.x += c0.x; c.y += c0.y; c.z += c0.z; c.w += c0.w;
             }
+            *pg = a;
+            if (!RMS) *pb = c;
+            else if (t == 0) *pb = make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
       }
@@ -402,26 +478,27 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_bwd_warp_kernel(
   }
   for (int c = threadIdx.x; c < H; c += blockDim.x) {
     if (partial) {
-      partial[(size_t)blockIdx.x * 2 * H + c] = nb_sums[c];
-      if (!RMS) partial[(size_t)blockIdx.x * 2 * H + H + c] = nb_sums[H + c];
+      partial[(size_t)blockIdx.x * 2 * H + c] = sums[c];
+      if (!RMS) partial[(size_t)blockIdx.x * 2 * H + H + c] = sums[H + c];
     } else {
-      if (dgamma) atomicAdd(dgamma + c, nb_sums[c]);
-      if (!RMS && dbeta) atomicAdd(dbeta + c, nb_sums[H + c]);
+      if (dgamma) atomicAdd(dgamma + c, sums[c]);
+      if (!RMS && dbeta) atomicAdd(dbeta + c, sums[H + c]);
     }
   }
 }
 
-// dgamma[c] += sum_b partial[b][0][c]; dbeta[c] += sum_b partial[b][1][c].
+// dgamma[c] (+)= sum_b partial[b][0][c]; dbeta[c] (+)= sum_b partial[b][1][c]. `store`: 0 adds to fp32 buffers, 1 writes fp32,
+// 2 writes bf16 (a gradient that starts here needs neither a zeroed buffer nor a cast).
 // A CTA owns 32 columns; its 32 x 32 threads split the nblk partial rows 32 ways (coalesced 128-byte reads), then
 // the 32 row-groups meet in shared memory. With hundreds of partial rows a one-thread-per-column loop is a chain of
 // dependent cache misses (47 us measured for H = 1024); this form takes a few microseconds.
 __global__ void __launch_bounds__(1024) norm_bwd_reduce_kernel(const float* __restrict__ partial,
-                                                               float* __restrict__ dgamma, float* __restrict__ dbeta,
-                                                               int nblk, int H) {
+                                                               void* __restrict__ dgamma, void* __restrict__ dbeta,
+                                                               int nblk, int H, int store) {
   __shared__ float red[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   const int which = blockIdx.y;  // 0 = gamma, 1 = beta
-  float* out = which == 0 ? dgamma : dbeta;
+  void* out = which == 0 ? dgamma : dbeta;
   if (!out) return;
   float s = 0.f;
   if (c < H) {
@@ -434,7 +511,9 @@ __global__ void __launch_bounds__(1024) norm_bwd_reduce_kernel(const float* __re
     float t = 0.f;
 #pragma unroll
     for (int y = 0; y < 32; ++y) t += red[y][threadIdx.x];
-    out[c] += t;
+    if (store == 2) reinterpret_cast<bf16*>(out)[c] = __float2bfloat16(t);
+    else if (store == 1) reinterpret_cast<float*>(out)[c] = t;
+    else reinterpret_cast<float*>(out)[c] += t;
   }
 }
 
@@ -475,28 +554,47 @@ static int norm_fwd_launch(const void* x, const void* gamma, const void* beta, v
   return 0;
 }
 
+template <typename T, int VPL, int NW, bool RMS>
+static int norm_bwd_ring_launch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                const void* dres, void* dx, float* dgamma, float* dbeta, float* partial, int rows, int H, int G,
+                                int* used, cudaStream_t st) {
+  auto kern = norm_bwd_ring_kernel<T, VPL, NW, RMS>;
+  const size_t ring = (size_t)(dres ? 2 * 3 : 3 * 2) * NW * VPL * 512, sums = (size_t)2 * H * sizeof(float);
+  const size_t smem = ring > sums ? ring : sums;
+  static bool configured = false;
+  if (!configured) {
+    TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    configured = true;
+  }
+  const int teams = NW / G, want = (rows + teams - 1) / teams, cap = sm_count();  // never above norm_bwd_grid(rows)
+  *used = want < cap ? want : cap;
+  kern<<<*used, NW * 32, smem, st>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)dres, (T*)dx, dgamma, dbeta,
+                                    partial, rows, H, G);
+  TB_CUDA_CHECK(cudaGetLastError());
+  return 0;
+}
+
 template <typename T, bool RMS>
 static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, const float* mean,
-                           const float* rstd, const void* dres, void* dx, float* dgamma,
-                           float* dbeta, float* partial, int rows, int H, cudaStream_t st) {
+                           const float* rstd, const void* dres, void* dx, void* dgamma_, void* dbeta_, float* partial, int rows,
+                           int H, int store, cudaStream_t st) {
   constexpr int N = Vec16<T>::N;
   if (H % N) TB_FAIL(TB_E_ARG, "norm: H=%d must be a multiple of %d", H, N);
+  float *dgamma = (float*)dgamma_, *dbeta = (float*)dbeta_;  // only touched by the kernels when there is no workspace
   int nvec = H / N;
   int grid = norm_bwd_grid(rows);
-  if (nvec <= 32 * 4) {  // eight vectors per lane would spill: wider rows keep the CTA-per-row kernel
-    // never more CTAs than the cap above: the workspace (also the fixed one of tb_norm_bwd_static) is sized for it
-    const int want = (rows + NORM_WARPS - 1) / NORM_WARPS;
-    const int cap = sm_count() * (nvec <= 32 ? 3 : 1);  // resident CTAs: 80 / 158 / 255 registers per thread
-    const int wgrid = want < (cap < grid ? cap : grid) ? want : (cap < grid ? cap : grid);
-    const size_t smem = (size_t)2 * H * sizeof(float);
-#define TB_NBW(VPL_)                                                                                           \
-  norm_bwd_warp_kernel<T, VPL_, RMS><<<wgrid, NORM_WARPS * 32, smem, st>>>(                                    \
-      (const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)dres, (T*)dx, dgamma, dbeta, partial, rows, H);
-    if (nvec <= 32) TB_NBW(1) else if (nvec <= 64) TB_NBW(2) else TB_NBW(4)
-#undef TB_NBW
+  if (H <= 8192) {
+    // 16 elements a lane and 16 warps, or 8 elements and 24 warps: whichever leaves fewer lanes without a vector
+    constexpr int V2 = 16 / N, V1 = 8 / N;
+    const int g2 = (nvec + 32 * V2 - 1) / (32 * V2), g1 = (nvec + 32 * V1 - 1) / (32 * V1);
+    const bool narrow = g1 <= 3 && g1 * V1 < g2 * V2;
+    int used = 0, r;
+    if (narrow) r = norm_bwd_ring_launch<T, V1, 24, RMS>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, g1, &used, st);
+    else r = norm_bwd_ring_launch<T, V2, 16, RMS>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, g2, &used, st);
+    if (r) return r;
     if (partial) {
       dim3 rgrid((H + 31) / 32, RMS ? 1 : 2);
-      norm_bwd_reduce_kernel<<<rgrid, dim3(32, 32), 0, st>>>(partial, dgamma, dbeta, wgrid, H);
+      norm_bwd_reduce_kernel<<<rgrid, dim3(32, 32), 0, st>>>(partial, dgamma_, dbeta_, used, H, store);
     }
     TB_CUDA_CHECK(cudaGetLastError());
     return 0;
@@ -509,12 +607,11 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
                                                              (const T*)dres, (T*)dx, dgamma,      \
                                                              dbeta, partial, rows, H);            \
   }
-  if (nvec <= 256) TB_NB(1) else if (nvec <= 1024) TB_NB(2) else if (nvec <= 4096) TB_NB(4) else
-    TB_FAIL(TB_E_ARG, "norm: H=%d too large", H);
+  if (nvec <= 4096) TB_NB(4) else TB_FAIL(TB_E_ARG, "norm: H=%d too large", H);
 #undef TB_NB
   if (partial) {
     dim3 rgrid((H + 31) / 32, RMS ? 1 : 2);
-    norm_bwd_reduce_kernel<<<rgrid, dim3(32, 32), 0, st>>>(partial, dgamma, dbeta, grid, H);
+    norm_bwd_reduce_kernel<<<rgrid, dim3(32, 32), 0, st>>>(partial, dgamma_, dbeta_, grid, H, store);
   }
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
@@ -543,6 +640,18 @@ TB_EXPORT long tb_norm_bwd_workspace(int rows, int H) {
   return (long)norm_bwd_grid(rows) * 2 * H;
 }
 
+namespace tb {
+static int norm_bwd_dispatch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                             const void* dres, void* dx, void* dgamma, void* dbeta, float* partial, int rows, int H, int rms,
+                             int dtype, int store, cudaStream_t st) {
+  if (dtype == 0)
+    return rms ? norm_bwd_launch<bf16, true>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, store, st)
+               : norm_bwd_launch<bf16, false>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, store, st);
+  return rms ? norm_bwd_launch<float, true>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, store, st)
+             : norm_bwd_launch<float, false>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, store, st);
+}
+}  // namespace tb
+
 // dgamma / dbeta are fp32 buffers that the kernel ACCUMULATES into (zero them for a fresh
 // gradient). dres (optional) is added to dx. `partial` is scratch memory of
 // tb_norm_bwd_workspace(rows, H) floats holding per-CTA partial sums that a second kernel
@@ -553,11 +662,16 @@ TB_EXPORT int tb_norm_bwd(const void* dy, const void* x, const void* gamma, cons
                           cudaStream_t st) {
   TB_ENSURE_DEVICE();
   if (rows <= 0) return 0;
-  if (dtype == 0)
-    return rms ? norm_bwd_launch<bf16, true>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, st)
-               : norm_bwd_launch<bf16, false>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, st);
-  return rms ? norm_bwd_launch<float, true>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, st)
-             : norm_bwd_launch<float, false>(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, st);
+  return norm_bwd_dispatch(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, rms, dtype, 0, st);
+}
+
+// The same with dgamma / dbeta WRITTEN in grad_dtype (0 bf16, 1 fp32), rows > 0; the workspace is required.
+TB_EXPORT int tb_norm_bwd_store(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                const void* dres, void* dx, void* dgamma, void* dbeta, float* partial, int rows, int H, int rms,
+                                int dtype, int grad_dtype, cudaStream_t st) {
+  TB_ENSURE_DEVICE();
+  if (rows <= 0 || !partial) TB_FAIL(TB_E_ARG, "norm_bwd_store: needs rows and a workspace");
+  return norm_bwd_dispatch(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, partial, rows, H, rms, dtype, grad_dtype == 0 ? 2 : 1, st);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -200,6 +200,41 @@ def test_norm_fwd_bwd(dtype, H, rms):
         assert _rel(b.grad, bf.grad) < tol
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H", [8, 264, 768, 1288, 2056, 8192])
+@pytest.mark.parametrize("rows", [1, 41, 2600])
+def test_norm_bwd_teams(dtype, H, rows):
+    """Every team size of the backward (1 to 16 warps a row), lanes without a vector, fewer rows than teams and several rows
+    a team, with a residual gradient and with gradients that accumulate. Tolerances: one bf16 rounding of the largest value
+    (2^-8) with room for the rounded inputs of the reference, and fp32 sums of up to 8192 terms."""
+    from torsh_b200.ops.norm import layer_norm_fork, rms_norm
+    torch.manual_seed(6)
+    tol = 2e-2 if dtype == torch.bfloat16 else 1e-4
+    x = torch.randn(rows, H, device=DEV, dtype=dtype, requires_grad=True)
+    w = (torch.randn(H, device=DEV) * 0.2 + 1).to(dtype).requires_grad_(True)
+    b = (torch.randn(H, device=DEV) * 0.1).to(dtype).requires_grad_(True)
+    dy, dr = (torch.randn(rows, H, device=DEV, dtype=dtype) for _ in range(2))
+    y, xx = layer_norm_fork(x, w, b, 1e-5)
+    grads = torch.autograd.grad((y, xx), (x, w, b), (dy, dr))
+    ref_in = [t.detach().float().requires_grad_(True) for t in (x, w, b)]
+    ref = torch.autograd.grad(torch.nn.functional.layer_norm(ref_in[0], (H,), ref_in[1], ref_in[2], 1e-5), ref_in, dy.float())
+    ref = (ref[0] + dr.float(), *ref[1:])
+    for g, r in zip(grads, ref):
+        assert g.dtype == dtype and _rel(g, r) < tol
+    w.main_grad = torch.ones(H, device=DEV)
+    b.main_grad = torch.ones(H, device=DEV)
+    y, xx = layer_norm_fork(x, w, b, 1e-5)
+    gx, gw, gb = torch.autograd.grad((y, xx), (x, w, b), (dy, dr), allow_unused=True)
+    assert gw is None and gb is None and _rel(gx, ref[0]) < tol
+    assert _rel(w.main_grad, ref[1] + 1) < tol and _rel(b.main_grad, ref[2] + 1) < tol
+    del w.main_grad
+    y = rms_norm(x, w, 1e-6)
+    gx, gw = torch.autograd.grad(y, (x, w), dy)
+    xf, wf = ref_in[:2]
+    rx, rw = torch.autograd.grad(xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * wf, (xf, wf), dy.float())
+    assert _rel(gx, rx) < tol and _rel(gw, rw) < tol
+
+
 # ------------------------------------------------------------------ softmax / cross-entropy
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("C", [1000, 4097, 50304])

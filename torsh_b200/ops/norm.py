@@ -12,6 +12,7 @@ from ._dispatch import F, I, P, aligned, call, dtype_code, kernel_ok
 
 _FWD = [P, P, P, P, P, P, I, I, F, I, I, P]
 _BWD = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
+_BWD_STORE = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
 
 
 _ws_cache: dict = {}
@@ -50,25 +51,38 @@ class _NormFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
-        rows, H = x2.shape
-        dy2 = aligned(dy.reshape(rows, H).to(x2.dtype))
-        dx = torch.empty_like(x2)
-        # gradients of weight / bias accumulate straight into fp32 `main_grad` buffers when the
-        # parameters carry them (flat mixed-precision storage); autograd then receives None
-        wmg, bmg = ctx.main_grads
-        dgamma = wmg.view(-1) if wmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
-        dbeta = None
-        if ctx.has_bias:
-            dbeta = bmg.view(-1) if bmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
-        ws = torch.empty(_workspace_elems(rows, H), dtype=torch.float32, device=x2.device)
-        call("tb_norm_bwd", _BWD, dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-             None, dx.data_ptr(), dgamma.data_ptr(), nv.ptr(dbeta), ws.data_ptr(), rows, H, int(ctx.rms),
-             dtype_code(x2), nv.stream_ptr())
+        return _norm_backward(ctx, dy, None)
+
+
+def _norm_backward(ctx, dy, dres):
+    x2, w, mean, rstd = ctx.saved_tensors
+    rows, H = x2.shape
+    dy2 = aligned(dy.reshape(rows, H).to(x2.dtype))
+    dr2 = aligned(dres.reshape(rows, H).to(x2.dtype)) if dres is not None else None
+    dx = torch.empty_like(x2)
+    wmg, bmg = ctx.main_grads
+    ws = torch.empty(_workspace_elems(rows, H), dtype=torch.float32, device=x2.device)
+    ptrs = (dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(), nv.ptr(dr2), dx.data_ptr())
+    if rows > 0 and wmg is None and bmg is None and (not ctx.has_bias or ctx.bdtype == ctx.wdtype):
+        # fresh gradients are written in their own dtype by the reduction: no zeroed fp32 buffers, no casts
+        gw = torch.empty(H, dtype=ctx.wdtype, device=x2.device)
+        gb = torch.empty(H, dtype=ctx.bdtype, device=x2.device) if ctx.has_bias else None
+        call("tb_norm_bwd_store", _BWD_STORE, *ptrs, gw.data_ptr(), nv.ptr(gb), ws.data_ptr(), rows, H, int(ctx.rms),
+             dtype_code(x2), dtype_code(gw), nv.stream_ptr())
         nv.launch_count += 1
-        gw = None if wmg is not None else dgamma.to(ctx.wdtype)
-        gb = None if (not ctx.has_bias or bmg is not None) else dbeta.to(ctx.bdtype)
         return dx.view(ctx.shape), gw, gb, None, None
+    # gradients of weight / bias accumulate straight into fp32 `main_grad` buffers when the
+    # parameters carry them (flat mixed-precision storage); autograd then receives None
+    dgamma = wmg.view(-1) if wmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
+    dbeta = None
+    if ctx.has_bias:
+        dbeta = bmg.view(-1) if bmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
+    call("tb_norm_bwd", _BWD, *ptrs, dgamma.data_ptr(), nv.ptr(dbeta), ws.data_ptr(), rows, H, int(ctx.rms),
+         dtype_code(x2), nv.stream_ptr())
+    nv.launch_count += 1
+    gw = None if wmg is not None else dgamma.to(ctx.wdtype)
+    gb = None if (not ctx.has_bias or bmg is not None) else dbeta.to(ctx.bdtype)
+    return dx.view(ctx.shape), gw, gb, None, None
 
 
 class _NormForkFn(torch.autograd.Function):
@@ -83,24 +97,7 @@ class _NormForkFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, dres):
-        x2, w, mean, rstd = ctx.saved_tensors
-        rows, H = x2.shape
-        dy2 = aligned(dy.reshape(rows, H).to(x2.dtype))
-        dr2 = aligned(dres.reshape(rows, H).to(x2.dtype)) if dres is not None else None
-        dx = torch.empty_like(x2)
-        wmg, bmg = ctx.main_grads
-        dgamma = wmg.view(-1) if wmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
-        dbeta = None
-        if ctx.has_bias:
-            dbeta = bmg.view(-1) if bmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
-        ws = torch.empty(_workspace_elems(rows, H), dtype=torch.float32, device=x2.device)
-        call("tb_norm_bwd", _BWD, dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-             nv.ptr(dr2), dx.data_ptr(), dgamma.data_ptr(), nv.ptr(dbeta), ws.data_ptr(), rows, H, int(ctx.rms),
-             dtype_code(x2), nv.stream_ptr())
-        nv.launch_count += 1
-        gw = None if wmg is not None else dgamma.to(ctx.wdtype)
-        gb = None if (not ctx.has_bias or bmg is not None) else dbeta.to(ctx.bdtype)
-        return dx.view(ctx.shape), gw, gb, None, None
+        return _norm_backward(ctx, dy, dres)
 
 
 def layer_norm_fork(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, eps: float = 1e-5):
