@@ -175,6 +175,156 @@ xent_kernel(const T* __restrict__ logits, const long* __restrict__ targets,
   }
 }
 
+// The same for rows of which two fit into shared memory (up to 55 296 bf16 or 27 648 fp32 columns): every thread copies its
+// own vectors of the next row (cp.async, no barrier) while it works on the current one, the row maximum and the exponent sum
+// meet in ONE block reduction of (maximum, sum) pairs, and nothing is re-read. Staging, sum and gradient of a row one after
+// the other, with two CTAs per SM to overlap them, took 242 us at 4096 x 50 304 bf16; this takes 178, against 126 us for
+// reading and writing the matrix at the copy rate and about 92 us of exponentials on the special-function units.
+__device__ __forceinline__ void xent_cp_async16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+__device__ __forceinline__ float2 exp_of_diff(float2 f, float2 minus_m) {   // __expf(f - m), two at a time
+  const float2 t = __fmul2_rn(__fadd2_rn(f, minus_m), make_float2(1.4426950408889634f, 1.4426950408889634f));
+  return make_float2(exp2f(t.x), exp2f(t.y));
+}
+
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS) xent_ring_kernel(const T* __restrict__ logits, const long* __restrict__ targets,
+                                                            float* __restrict__ loss_rows, float* __restrict__ lse_rows,
+                                                            T* dlogits, int rows, int C, long ld, float scale,
+                                                            long ignore_index) {
+  constexpr int N = Vec16<T>::N;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  __shared__ float2 red[2][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nvec = (C + N - 1) / N, nld = (int)(ld / N);   // vectors with valid columns, vectors of the whole row
+  auto buf = [&](int b) { return reinterpret_cast<T*>(smem_raw) + (size_t)b * nvec * N; };
+  auto request = [&](int row, int b) {
+    if (row < rows) {
+      const T* xr = logits + (size_t)row * ld;
+      for (int v = tid; v < nvec; v += THREADS) xent_cp_async16(buf(b) + v * N, xr + (size_t)v * N);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  request(blockIdx.x, 0);
+  int b = 0;
+  for (int row = blockIdx.x; row < rows; row += gridDim.x, b ^= 1) {
+    request(row + gridDim.x, b ^ 1);
+    const long tgt = targets[row];
+    const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= C;
+    if (ignored && tgt != ignore_index && tid == 0) report_bad_index();   // a target outside [0, C) that is not the ignore value
+    // read before anything of this row is overwritten (the gradient may be in place)
+    const float xt = tid == 0 && !ignored ? to_f<T>(logits[(size_t)row * ld + tgt]) : 0.f;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    const T* srow = buf(b);
+    // whole vectors carry no column tests; the last, ragged one is finished by one thread
+    const int nfull = C / N;
+    const bool tail = nfull < nvec && tid == nfull % THREADS;
+    float m = -FLT_MAX;
+    for (int v = tid; v < nfull; v += THREADS) {
+      Vec16<T> t;
+      t.load(srow + v * N);
+      float f[N];
+      t.get(f);
+#pragma unroll
+      for (int j = 0; j < N; ++j) m = fmaxf(m, f[j]);
+    }
+    if (tail)
+      for (int i = nfull * N; i < C; ++i) m = fmaxf(m, to_f<T>(srow[i]));
+    float2 s2 = make_float2(0.f, 0.f);
+    const float2 nm = make_float2(-m, -m);
+#pragma unroll 2
+    for (int v = tid; v < nfull; v += THREADS) {
+      Vec16<T> t;
+      t.load(srow + v * N);
+      float f[N];
+      t.get(f);
+#pragma unroll
+      for (int j = 0; j < N; j += 2) s2 = __fadd2_rn(s2, exp_of_diff(make_float2(f[j], f[j + 1]), nm));
+    }
+    if (tail)
+      for (int i = nfull * N; i < C; ++i) s2.x += __expf(to_f<T>(srow[i]) - m);
+    float s = s2.x + s2.y;
+    {
+      const float mw = warp_max(m);
+      s = warp_sum(s * __expf(m - mw));
+      if (lane == 0) red[b][warp] = make_float2(mw, s);   // two sets: the next row's sums do not wait for this row's readers
+      __syncthreads();
+      const float2 e = lane < THREADS / 32 ? red[b][lane] : make_float2(-FLT_MAX, 0.f);
+      m = warp_max(e.x);
+      s = warp_sum(e.y * __expf(e.x - m));
+    }
+    const float lse = m + __logf(s);
+    if (tid == 0) {
+      loss_rows[row] = lse - (ignored ? lse : xt);
+      if (lse_rows) lse_rows[row] = lse;
+    }
+    if (dlogits) {
+      T* dr = dlogits + (size_t)row * ld;
+      const float sc = ignored ? 0.f : scale;
+      const float2 nl = make_float2(-lse, -lse), sc2 = make_float2(sc, sc);
+      const int tvec = ignored ? -1 : (int)(tgt / N), tj = (int)(tgt - (long)tvec * N);
+#pragma unroll 2
+      for (int v = tid; v < nfull; v += THREADS) {
+        Vec16<T> t;
+        t.load(srow + v * N);
+        float f[N], o[N];
+        t.get(f);
+#pragma unroll
+        for (int j = 0; j < N; j += 2) {
+          const float2 pr = exp_of_diff(make_float2(f[j], f[j + 1]), nl);
+          o[j] = pr.x;
+          o[j + 1] = pr.y;
+        }
+        if (v == tvec) {
+#pragma unroll
+          for (int j = 0; j < N; ++j)
+            if (j == tj) o[j] -= 1.f;
+        }
+#pragma unroll
+        for (int j = 0; j < N; j += 2) {
+          const float2 pr = __fmul2_rn(make_float2(o[j], o[j + 1]), sc2);
+          o[j] = pr.x;
+          o[j + 1] = pr.y;
+        }
+        t.set(o);
+        t.store(dr + (size_t)v * N);
+      }
+      // the ragged vector (staged by its thread) and the padding
+      for (int v = nfull + (tid - nfull % THREADS + THREADS) % THREADS; v < nld; v += THREADS) {
+        float o[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const int i = v * N + j;
+          o[j] = i < C ? (__expf(to_f<T>(srow[i]) - lse) - (v == tvec && j == tj ? 1.f : 0.f)) * sc : 0.f;
+        }
+        Vec16<T> t;
+        t.set(o);
+        t.store(dr + (size_t)v * N);
+      }
+    }
+  }
+}
+
+// One CTA: valid = max(1, rows that are not ignored); loss = sum of the row losses * factor, or / valid when `mean`.
+__global__ void __launch_bounds__(1024) xent_mean_kernel(const float* __restrict__ loss_rows, const long* __restrict__ targets,
+                                                         int rows, long ignore_index, int mean, float factor,
+                                                         float* __restrict__ loss, float* __restrict__ valid) {
+  __shared__ float scratch[32];
+  float s = 0.f, n = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < rows; i += 1024) {
+    s += loss_rows[i];
+    n += targets[i] != ignore_index ? 1.f : 0.f;
+  }
+  s = block_sum(s, scratch);
+  n = fmaxf(block_sum(n, scratch), 1.f);
+  if (threadIdx.x == 0) {
+    *valid = n;
+    *loss = mean ? s / n : s * factor;
+  }
+}
+
 template <typename K>
 static int set_smem(K kern, size_t bytes) {
   if (bytes > 48 * 1024) TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -207,6 +357,25 @@ static int xent_launch(const void* logits, const long* targets, float* loss_rows
                        void* dlogits, int rows, int C, long ld, float scale, long ignore_index,
                        cudaStream_t st) {
   size_t bytes = (size_t)C * sizeof(T);
+  const size_t ring = 2 * ((bytes + 15) / 16 * 16);
+  const bool aligned = !((uintptr_t)logits & 15) && !((uintptr_t)dlogits & 15) && (ld * sizeof(T)) % 16 == 0;
+  if (aligned && ring <= 216 * 1024) {
+    // about six vectors a thread; as many CTAs per SM as threads (2048) and shared memory (216 KB) allow
+    const int nvec = (int)(bytes / 16), th = nvec >= 3072 ? 1024 : nvec >= 768 ? 512 : nvec >= 192 ? 256 : 128;
+    const int fit = (int)((size_t)216 * 1024 / (ring + 1024)), by_thr = 2048 / th;
+    const int per_sm = fit < 1 ? 1 : fit < by_thr ? fit : by_thr;
+    const int grid = rows < sm_count() * per_sm ? rows : sm_count() * per_sm;
+#define TB_XR(TH_)                                                                                                             \
+  {                                                                                                                            \
+    auto k = xent_ring_kernel<T, TH_>;                                                                                         \
+    if (int r = set_smem(k, ring)) return r;                                                                                   \
+    k<<<grid, TH_, ring, st>>>((const T*)logits, targets, loss_rows, lse_rows, (T*)dlogits, rows, C, ld, scale, ignore_index); \
+  }
+    if (th == 1024) TB_XR(1024) else if (th == 512) TB_XR(512) else if (th == 256) TB_XR(256) else TB_XR(128)
+#undef TB_XR
+    TB_CUDA_CHECK(cudaGetLastError());
+    return 0;
+  }
   bool cache = bytes <= SM_MAX_CACHE_BYTES;
   int grid = rows < sm_count() * 4 ? rows : sm_count() * 4;
   int threads = C >= 4096 ? SM_THREADS : (C >= 1024 ? 256 : 128);
@@ -261,6 +430,16 @@ TB_EXPORT int tb_cross_entropy(const void* logits, const long* targets, float* l
   if (ld < C) TB_FAIL(TB_E_ARG, "tb_cross_entropy: ld (%ld) < C (%d)", ld, C);
   return dtype == 0 ? xent_launch<bf16>(logits, targets, loss_rows, lse_rows, dlogits, rows, C, ld, scale, ignore_index, st)
                     : xent_launch<float>(logits, targets, loss_rows, lse_rows, dlogits, rows, C, ld, scale, ignore_index, st);
+}
+
+// loss = mean of the row losses over the rows that are not ignored, or (mean = 0) their sum times factor; valid = the number of
+// those rows, at least 1.
+TB_EXPORT int tb_cross_entropy_mean(const float* loss_rows, const long* targets, int rows, long ignore_index, int mean,
+                                    float factor, float* loss, float* valid, cudaStream_t st) {
+  TB_ENSURE_DEVICE();
+  xent_mean_kernel<<<1, 1024, 0, st>>>(loss_rows, targets, rows < 0 ? 0 : rows, ignore_index, mean, factor, loss, valid);
+  TB_CUDA_CHECK(cudaGetLastError());
+  return 0;
 }
 
 int tb_set_check_word_xent(int* word) {

@@ -282,6 +282,35 @@ def test_cross_entropy_padded_vocab(dtype):
     assert _rel(lg2.grad[:, :V], lf2.grad) < tol
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V,ld", [(1, 8), (130, 136), (1000, 1000), (4093, 4096), (27648, 27648), (27649, 27656), (55296, 55296)])
+@pytest.mark.parametrize("rows", [1, 333])
+def test_cross_entropy_row_sizes(dtype, V, ld, rows):
+    """Both sides of the sizes at which two rows stop fitting into shared memory, every CTA width, remainders of columns,
+    several rows a CTA, an ignored and a largest target, gradients in place and not. Gradients are one bf16 (fp32) rounding of
+    values computed in fp32; the loss is a mean of fp32 row losses."""
+    from torsh_b200.ops.softmax import cross_entropy
+    torch.manual_seed(8)
+    x = (torch.randn(rows, ld, device=DEV) * 2).to(dtype)
+    tg = torch.randint(0, V, (rows,), device=DEV)
+    tg[0] = V - 1
+    if rows > 1:
+        tg[5] = -100
+    ref_in = x.float()[:, :V].clone().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(ref_in, tg)
+    ref.backward()
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-4
+    for inplace in (False, True):
+        lg = x.clone().requires_grad_(True)
+        y = lg * 1.0
+        loss = cross_entropy(y, tg, num_classes=V, inplace_grad=inplace)
+        loss.backward()
+        assert abs(loss.item() - ref.item()) <= 1e-4 * max(1.0, abs(ref.item()))
+        assert _rel(lg.grad[:, :V], ref_in.grad) < tol and lg.grad[:, V:].abs().sum().item() == 0.0
+    neg = cross_entropy(x, tg.clamp(min=0), num_classes=V, root_scale=-2.0)
+    assert abs(neg.item() + 2 * torch.nn.functional.cross_entropy(ref_in.detach(), tg.clamp(min=0)).item()) < 1e-3 * max(1.0, abs(neg.item()))
+
+
 # ------------------------------------------------------------------ elementwise / reduce / embedding / rope
 def test_unary_binary_reduce():
     from torsh_b200.ops import elementwise as ew

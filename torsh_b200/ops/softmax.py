@@ -46,6 +46,7 @@ def log_softmax(x: torch.Tensor, dim: int = -1) -> torch.Tensor:
 
 
 _XENT = [P, P, P, P, P, I, I, L, F, L, I, P]
+_XENT_MEAN = [P, P, I, L, I, F, P, P, P]
 
 
 class _CrossEntropyFn(torch.autograd.Function):
@@ -58,7 +59,6 @@ class _CrossEntropyFn(torch.autograd.Function):
         assert lg.stride(1) == 1 and lg.data_ptr() % 16 == 0 and (lg.stride(0) * lg.element_size()) % 16 == 0
         rows = lg.shape[0]
         tg = targets.reshape(-1).contiguous().to(torch.int64)
-        valid = (tg != ignore_index).sum().clamp(min=1).to(torch.float32)
         loss_rows = torch.empty(rows, dtype=torch.float32, device=logits.device)
         need_grad = logits.requires_grad
         dl = (lg if inplace_grad else torch.empty_like(lg)) if need_grad else None
@@ -69,10 +69,10 @@ class _CrossEntropyFn(torch.autograd.Function):
         kscale = 1.0 if root_scale is None else float(root_scale) / rows
         call("tb_cross_entropy", _XENT, lg.data_ptr(), tg.data_ptr(), loss_rows.data_ptr(), None, nv.ptr(dl), rows,
              num_classes, lg.stride(0), kscale, ignore_index, dtype_code(lg), nv.stream_ptr())
-        if root_scale is None:
-            loss = loss_rows.sum() / valid
-        else:
-            loss = loss_rows.sum() * (float(root_scale) / rows)
+        # the mean (or root_scale / rows times the sum) and the number of counted rows in one launch
+        loss, valid = (torch.empty((), dtype=torch.float32, device=logits.device) for _ in range(2))
+        call("tb_cross_entropy_mean", _XENT_MEAN, loss_rows.data_ptr(), tg.data_ptr(), rows, ignore_index,
+             int(root_scale is None), kscale, loss.data_ptr(), valid.data_ptr(), nv.stream_ptr())
         if need_grad:
             ctx.save_for_backward(dl, valid)
         ctx.shape, ctx.root = logits.shape, root_scale is not None
