@@ -235,6 +235,28 @@ def test_norm_bwd_teams(dtype, H, rows):
     assert _rel(gx, rx) < tol and _rel(gw, rw) < tol
 
 
+@pytest.mark.parametrize("B,S,H,D", [(1, 5, 1, 64), (2, 130, 3, 64), (2, 77, 5, 128), (1, 256, 8, 128)])
+def test_rope_attention_packed_matches_separate_ops(B, S, H, D):
+    """The packed rotation and attention against rope() and flash_attention() on slices of the same projection: the rotations
+    round the same values in the same way, so outputs agree exactly and gradients up to the order of the fp32 dQ sums."""
+    from torsh_b200.ops.attention import flash_attention, rope_flash_attention_qkvpacked
+    from torsh_b200.ops.elementwise import rope
+    torch.manual_seed(9)
+    E = H * D
+    qkv = torch.randn(B * S, 3 * E, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    dy = torch.randn(B * S, E, device=DEV, dtype=torch.bfloat16)
+    out = rope_flash_attention_qkvpacked(qkv, B, S, H, D, 10000.0)
+    (g,) = torch.autograd.grad(out, qkv, dy)
+    q, k, v = (qkv[:, i * E:(i + 1) * E].reshape(B, S, H, D) for i in range(3))
+    ref = flash_attention(rope(q, 10000.0), rope(k, 10000.0), v, causal=True).reshape(B * S, E)
+    (rg,) = torch.autograd.grad(ref, qkv, dy)
+    assert torch.equal(out, ref)
+    assert _rel(g, rg) < 1e-2
+    with torch.no_grad():   # a strided view is taken, too
+        wide = torch.cat([qkv, qkv], 1)
+        assert torch.equal(rope_flash_attention_qkvpacked(wide[:, :3 * E], B, S, H, D, 10000.0), ref)
+
+
 # ------------------------------------------------------------------ softmax / cross-entropy
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("C", [1000, 4097, 50304])

@@ -89,11 +89,7 @@ class LlamaBlock(nn.Module):
         cfg, H, D = self.cfg, self.local_heads, self.cfg.head_dim
         h, x = norm_ops.rms_norm_fork(x, self.input_norm.weight, cfg.rms_eps)
         qkv = self.qkv(h)                                        # [B*S, 3*H*D] (all tokens, local heads)
-        E_loc = H * D
-        q = ew.rope(qkv[:, :E_loc].reshape(B, S, H, D), cfg.rope_theta)
-        k = ew.rope(qkv[:, E_loc:2 * E_loc].reshape(B, S, H, D), cfg.rope_theta)
-        v = qkv[:, 2 * E_loc:].reshape(B, S, H, D)
-        ctx = attn_ops.flash_attention(q, k, v, causal=True).reshape(B * S, E_loc)
+        ctx = attn_ops.rope_flash_attention_qkvpacked(qkv, B, S, H, D, cfg.rope_theta)
         x = self.o(ctx, residual=x)
         h, x = norm_ops.rms_norm_fork(x, self.post_attn_norm.weight, cfg.rms_eps)
         return self.down(ew.swiglu(self.gate_up(h)), residual=x)

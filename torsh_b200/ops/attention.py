@@ -11,7 +11,7 @@ import math
 import torch
 
 from .. import _native as nv
-from ._dispatch import F, I, L, P, call, kernel_ok
+from ._dispatch import F, I, L, P, aligned, call, kernel_ok
 
 _FWD = [P, P, P, P, P, I, I, I, I, L, L, L, F, I, P, P]
 _BWD = [P] * 11 + [I, I, I, I, L, L, L, L, L, F, I, P, P]
@@ -59,6 +59,39 @@ class _FlashQKVPacked(torch.autograd.Function):
         _bwd(qkv[:, :E], qkv[:, E:2 * E], qkv[:, 2 * E:], out, dout, lse, dqkv[:, :E], dqkv[:, E:2 * E],
              dqkv[:, 2 * E:], B, S, H, D, st, st, dqkv.stride(0), scale, causal)
         return dqkv, None, None, None, None, None, None
+
+
+_ROPE_QKV = [P, P, L, I, I, I, L, L, F, I, P]
+
+
+class _RopeFlashQKVPacked(torch.autograd.Function):
+    """Rotary positions on the q and k bands of ``qkv [B*S, 3*H*D]``, then attention -> ``[B*S, H*D]``."""
+
+    @staticmethod
+    def forward(ctx, qkv, B, S, H, D, base, causal, scale):
+        E = H * D
+        qkv = aligned(qkv)
+        rot = torch.empty_like(qkv)
+        call("tb_rope_qkv", _ROPE_QKV, qkv.data_ptr(), rot.data_ptr(), B * S, S, H, D, 3 * E, 3 * E, float(base), 0, nv.stream_ptr())
+        out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
+        lse = torch.empty(B * H * S, dtype=torch.float32, device=qkv.device)
+        _fwd(rot[:, :E], rot[:, E:2 * E], rot[:, 2 * E:], out, lse, B, S, H, D, 3 * E, 3 * E, scale, causal)
+        ctx.save_for_backward(rot, out, lse)
+        ctx.dims = (B, S, H, D, base, causal, scale)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        rot, out, lse = ctx.saved_tensors
+        B, S, H, D, base, causal, scale = ctx.dims
+        E = H * D
+        dout = aligned(dout)
+        dqkv = torch.empty_like(rot)
+        _bwd(rot[:, :E], rot[:, E:2 * E], rot[:, 2 * E:], out, dout, lse, dqkv[:, :E], dqkv[:, E:2 * E], dqkv[:, 2 * E:],
+             B, S, H, D, 3 * E, 3 * E, 3 * E, scale, causal)
+        # the gradient of a rotation is the rotation back; dq and dk are turned where they lie
+        call("tb_rope_qkv", _ROPE_QKV, dqkv.data_ptr(), dqkv.data_ptr(), B * S, S, H, D, 3 * E, 3 * E, float(base), 1, nv.stream_ptr())
+        return dqkv, None, None, None, None, None, None, None
 
 
 class _FlashSeparate(torch.autograd.Function):
@@ -118,3 +151,15 @@ def flash_attention_qkvpacked(qkv: torch.Tensor, B: int, S: int, H: int, D: int,
         return _FlashQKVPacked.apply(qkv, B, S, H, D, causal, scale)
     q, k, v = (qkv[:, i * E:(i + 1) * E].reshape(B, S, H, D) for i in range(3))
     return _sdpa_reference(q, k, v, causal, scale).reshape(B * S, E)
+
+
+def rope_flash_attention_qkvpacked(qkv: torch.Tensor, B: int, S: int, H: int, D: int, rope_base: float = 10000.0,
+                                   causal: bool = True, scale: float | None = None) -> torch.Tensor:
+    """:func:`flash_attention_qkvpacked` with rotary positions (:func:`~torsh_b200.ops.elementwise.rope`) on q and k first."""
+    E = H * D
+    if kernel_ok(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and qkv.shape == (B * S, 3 * E):
+        return _RopeFlashQKVPacked.apply(qkv, B, S, H, D, rope_base, causal, 1.0 / math.sqrt(D) if scale is None else scale)
+    from .elementwise import rope
+    q = rope(qkv[:, :E].reshape(B, S, H, D), rope_base)
+    k = rope(qkv[:, E:2 * E].reshape(B, S, H, D), rope_base)
+    return flash_attention(q, k, qkv[:, 2 * E:].reshape(B, S, H, D), causal=causal, scale=scale).reshape(B * S, E)
