@@ -235,6 +235,32 @@ def test_norm_bwd_teams(dtype, H, rows):
     assert _rel(gx, rx) < tol and _rel(gw, rw) < tol
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S", [129, 640, 1100])
+def test_flash_attention_many_tiles(D, causal, S):
+    """More tiles than SMs (two CTAs per SM), row maxima that keep growing along the keys (the running output is rescaled in
+    most blocks), and rows whose largest score comes first (never rescaled). P, O and the gradients carry bf16 roundings, as
+    in the smaller tests; the tolerance is theirs."""
+    from torsh_b200.ops.attention import _sdpa_reference, flash_attention
+    torch.manual_seed(13)
+    B, H = 5, 32
+    q, k, v, do = (torch.randn(B, S, H, D, device=DEV, dtype=torch.bfloat16) for _ in range(4))
+    ramp = torch.linspace(0.2, 6.0, S, device=DEV).view(1, S, 1, 1)
+    k[: B // 2] = (k[: B // 2].float() * ramp).to(k.dtype)
+    k[B // 2:] = (k[B // 2:].float() * ramp.flip(1)).to(k.dtype)
+    a = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out = flash_attention(*a, causal=causal)
+    grads = torch.autograd.grad(out, a, do)
+    for b in range(B):
+        r = [t[b:b + 1].float().requires_grad_(True) for t in (q, k, v)]
+        ref = _sdpa_reference(*r, causal, D ** -0.5)
+        rg = torch.autograd.grad(ref, r, do[b:b + 1].float())
+        assert _rel(out[b:b + 1], ref) < 2e-2
+        for g, x in zip(grads, rg):
+            assert ((g[b:b + 1].float() - x).norm() / x.norm()).item() < 2e-2
+
+
 @pytest.mark.parametrize("B,S,H,D", [(1, 5, 1, 64), (2, 130, 3, 64), (2, 77, 5, 128), (1, 256, 8, 128)])
 def test_rope_attention_packed_matches_separate_ops(B, S, H, D):
     """The packed rotation and attention against rope() and flash_attention() on slices of the same projection: the rotations
