@@ -779,7 +779,8 @@ TB_EXPORT int tb_bn_apply(const void* x, const void* res, void* y, const float* 
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
-// dgamma / dbeta (fp32 [C]) are accumulated into; dres may be null; y is read only when relu != 0.
+// dgamma / dbeta (fp32 [C]) are accumulated into, or null: sums [2*C] then holds dbeta and dgamma. dres may be null; y is read
+// only when relu != 0.
 TB_EXPORT int tb_bn_bwd(const void* dy, const void* y, const void* x, const float* mean, const float* rstd,
                         const float* gamma, const float* beta, float* sums, void* dx, void* dres, float* dgamma,
                         float* dbeta, long rows, int C, int relu, cudaStream_t st) {
@@ -812,7 +813,7 @@ TB_EXPORT int tb_bn_bwd(const void* dy, const void* y, const void* x, const floa
     bn_bwd_reduce_kernel<<<grid, dim3(32, 8), 0, st>>>((const bf16*)dy, (const bf16*)y, (const bf16*)x, mean, rstd, sums, rows, C, relu, rpb);
     bn_bwd_apply_kernel<<<grid_1d(rows * (C >> 3)), 256, 0, st>>>((const bf16*)dy, (const bf16*)y, (const bf16*)x, mean, rstd, gamma, sums, (bf16*)dx, (bf16*)dres, rows, C, relu);
   }
-  bn_param_grad_kernel<<<(C + 255) / 256, 256, 0, st>>>(sums, dgamma, dbeta, C);
+  if (dgamma && dbeta) bn_param_grad_kernel<<<(C + 255) / 256, 256, 0, st>>>(sums, dgamma, dbeta, C);
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -568,28 +568,49 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (!*abort_flag && !wait_flag_ge_gpu(p.ag_ready + m_t, ag_epoch, p.status)) *abort_flag = 1;
           fence_proxy_async_all();
         }
+        // Convolutions: tile and tap coordinates are kept across the K blocks. Divided out anew for every copy they made the
+        // producer thread the bottleneck (3 x 3, 64 -> 64 channels, batch 64 of 56 x 56: forward 56 -> 44 us and input gradient
+        // 72 -> 50 us together with 64-wide tiles, weight gradient 56 -> 48).
+        int cv_n0 = 0, cv_h0 = 0, tap = 0, cc = 0, a_chunks = BM / 64, b_chunks = BN / 64;
+        int b_ci[BN / 64], b_kh[BN / 64], b_kw[BN / 64];
+        if (A_MAJOR == 0 && p.conv) {
+          int valid;
+          long base_row;
+          conv_tile(p, m_t, cv_n0, cv_h0, base_row, valid);
+          tap = kb0 / p.cv_cchunks;
+          cc = kb0 - tap * p.cv_cchunks;
+        } else if (A_MAJOR == 1 && p.conv == 3) {
+          tap = kb0 / p.cv_tiles_h;              // image group and row group of the pixel block
+          cc = kb0 - tap * p.cv_tiles_h;
+          a_chunks = min(BM / 64, (p.M - m_t * BM + 63) >> 6);
+          const int cin = p.N / 9;
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c) {
+            const int col = n_t * BN + c * 64, t9 = col / cin;
+            if (t9 >= 9) b_chunks = min(b_chunks, c);   // nothing is loaded past the last tap (those rows stay zero)
+            b_ci[c] = col - t9 * cin;
+            b_kh[c] = t9 / 3 - 1;
+            b_kw[c] = t9 - t9 / 3 * 3 - 1;
+          }
+        }
         for (int kb = kb0; kb < kb1; ++kb) {
           if (p.wg_on && B_MAJOR == 1)
             wg_wait(p.wg_b_off + (long)kb * BK * p.wg_ldb_bytes, p.wg_b_off + (long)min(p.K, (kb + 1) * BK) * p.wg_ldb_bytes);
           if (*abort_flag || !mbar_wait(&empty[s], phase ^ 1, abort_flag, p.status, TB_ERR_WAIT_EMPTY)) break;
           uint8_t* sa = smem + s * L::STAGE_BYTES;
           uint8_t* sb = sa + A_TILE_BYTES;
-          mbar_expect_tx(&full[s], p.conv == 3 ? (uint32_t)(p.cv_a_bytes * (BM / 64 + BN / 64))
+          mbar_expect_tx(&full[s], p.conv == 3 ? (uint32_t)(p.cv_a_bytes * (a_chunks + b_chunks))
                                   : p.conv ? (uint32_t)(p.cv_a_bytes + L::B_TILE_BYTES) : (uint32_t)L::STAGE_BYTES);
           if (A_MAJOR == 0 && p.conv) {
-            const int tap = kb / p.cv_cchunks, cc = kb - tap * p.cv_cchunks;
             const int kh = tap / 3, kw = tap - kh * 3;
-            int n0, h0, valid;
-            long base_row;
-            conv_tile(p, m_t, n0, h0, base_row, valid);
-            tma_load_4d(sa, &map_a, &full[s], cc * 64, kw - 1, h0 + kh - 1, n0);
+            tma_load_4d(sa, &map_a, &full[s], cc * 64, kw - 1, cv_h0 + kh - 1, cv_n0);
           } else if (A_MAJOR == 0) {
             tma_load_2d(sa, &map_a, &full[s], kb * BK, m_t * BM);
           } else if (p.conv == 3) {
-            const int it = kb / p.cv_tiles_h, ht = kb - it * p.cv_tiles_h;
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
-              tma_load_4d(sa + c * (64 * BK * 2), &map_a, &full[s], m_t * BM + c * 64, 0, ht * p.cv_TH, it * p.cv_TN);
+              if (c < a_chunks)
+                tma_load_4d(sa + c * (64 * BK * 2), &map_a, &full[s], m_t * BM + c * 64, 0, cc * p.cv_TH, tap * p.cv_TN);
           } else {
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
@@ -598,20 +619,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (B_MAJOR == 0) {
             tma_load_2d(sb, &map_b, &full[s], kb * BK, n_t * BN);
           } else if (p.conv == 3) {
-            const int it = kb / p.cv_tiles_h, ht = kb - it * p.cv_tiles_h;
-            const int cin = p.N / 9;
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c) {
-              const int col = n_t * BN + c * 64;
-              const int tap = min(col / cin, 8);          // chunks past the last tap load something harmless
-              const int ci0 = col - (col / cin) * cin;
-              const int kh = tap / 3, kw = tap - kh * 3;
-              tma_load_4d(sb + c * (64 * BK * 2), &map_b, &full[s], ci0, kw - 1, ht * p.cv_TH + kh - 1, it * p.cv_TN);
-            }
+            for (int c = 0; c < BN / 64; ++c)
+              if (c < b_chunks)
+                tma_load_4d(sb + c * (64 * BK * 2), &map_b, &full[s], b_ci[c], b_kw[c], cc * p.cv_TH + b_kh[c], tap * p.cv_TN);
           } else if (p.conv == 2) {
             // input gradient: weights [Cout, 9 * Cin] read MN-major; tap t of the gradient pairs with tap 8 - t of the
             // forward filter, whose Cin columns start at (8 - t) * Cin; the K rows are the Cout chunk
-            const int tap = kb / p.cv_cchunks, cc = kb - tap * p.cv_cchunks;
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
               tma_load_2d(sb + c * (64 * BK * 2), &map_b, &full[s], (8 - tap) * p.N + n_t * BN + c * 64, cc * BK);
@@ -619,6 +633,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
               tma_load_2d(sb + c * (64 * BK * 2), &map_b, &full[s], n_t * BN + c * 64, kb * BK);
+          }
+          if (p.conv && ++cc == (p.conv == 3 ? p.cv_tiles_h : p.cv_cchunks)) {
+            cc = 0;
+            ++tap;
           }
           if (++s == STAGES) {
             s = 0;
@@ -1002,7 +1020,7 @@ static int route(const GemmArgs& a, int& bn, int& S) {
   const long t256 = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
   const long m128 = (a.M + 127) / 128, t128 = m128 * ((a.N + 127) / 128);
   int best = ROUTE_ONE;
-  double t = 5.0 + waves(t128, sms) * fmax(kb * 0.25 * mn, 1.9);
+  double t = 5.0 + waves(t128, sms) * fmax(kb * (a.N <= 64 ? 0.18 : 0.25) * mn, 1.9);
   if (pair) {
     const double tp = 5.3 + waves(t256, sms / 2) * fmax(kb * 0.30 + 0.6, 2.9);
     if (tp < t) {
@@ -1037,6 +1055,7 @@ TB_EXPORT int tb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, 
                            const void* residual, int ldr, void* preact, const void* aux, int flags,
                            int split_k, int bn, int* status, cudaStream_t stream) {
   TB_ENSURE_DEVICE();
+  if (bn != 0 && bn != 128 && bn != 256) TB_FAIL(TB_E_ARG, "tb_gemm_bf16: bn must be 128 or 256");
   GemmArgs ga{A, B, D, M, N, K, a_major, b_major, lda, ldb, ldd, bias, residual, ldr, preact, aux, flags, split_k, status};
   if (bn == 0 && split_k >= 0 && !g_dynamic_tiles) {
     int S = 1;
@@ -1126,8 +1145,10 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     // leaves SMs idle.
     long t256 = (long)((M + BM - 1) / BM) * ((N + 255) / 256) * split_k;
     bn = (N > 128 && t256 >= sm_count()) ? 256 : 128;
+    // narrow outputs (64-channel convolutions): nothing is loaded or multiplied for columns that do not exist
+    if (N <= 64 && (tp.kind == 0 || tp.kind == 3)) bn = 64;
   }
-  if (bn != 128 && bn != 256) TB_FAIL(TB_E_ARG, "tb_gemm_bf16: bn must be 128 or 256");
+  if (bn != 64 && bn != 128 && bn != 256) TB_FAIL(TB_E_ARG, "tb_gemm_bf16: bn must be 128 or 256");
 
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
@@ -1305,7 +1326,8 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     return launch_gemm<128, 0, 1, 4, 3>(ma, mb, om, p, stream);
   }
   if (bn == 256) TB_DISPATCH(256, 4);
-  else TB_DISPATCH(128, 6);
+  else if (bn == 128) TB_DISPATCH(128, 6);
+  else TB_DISPATCH(64, 8);
 #undef TB_DISPATCH
   TB_FAIL(TB_E_ARG, "tb_gemm_bf16: unsupported major combination");
 }

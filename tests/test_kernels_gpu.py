@@ -145,6 +145,58 @@ def test_gemm_pair_tiles_and_epilogues(shape, majors):
     nv.check_status()
 
 
+@pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("shape", [(40000, 64, 256), (39992, 8, 64), (30000, 56, 72)])
+def test_gemm_narrow_outputs(shape, majors):
+    """At most 64 output columns and many rows: the 64-wide tiles, whole and ragged, with bias and residual. One bf16 rounding."""
+    from torsh_b200.ops.gemm import gemm
+    torch.manual_seed(14)
+    M, N, K = shape
+    am, bm = majors
+    a = torch.randn((K, M) if am else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if bm else (N, K), device=DEV, dtype=torch.bfloat16) / K ** 0.5
+    bias, res = torch.randn(N, device=DEV, dtype=torch.bfloat16), torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    u = (a.float().t() if am else a.float()) @ (b.float() if bm else b.float().t())
+    assert _rel_elem(gemm(a, b, a_major=am, b_major=bm), u) < 1e-2
+    assert _rel_elem(gemm(a, b, a_major=am, b_major=bm, bias=bias, residual=res), u + bias.float() + res.float()) < 1e-2
+
+
+@pytest.mark.parametrize("n,hw,ci,co", [(3, 9, 64, 64), (2, 56, 64, 128), (5, 7, 128, 64), (1, 64, 64, 192), (9, 14, 192, 64)])
+def test_conv3x3_tiles_and_chunks(n, hw, ci, co):
+    """Implicit 3x3 convolution and both gradients where a tile has channel chunks that do not exist (64 filters in a 128-row
+    tile, a last column tile of fewer than four taps), several images a tile and ragged row blocks. Inputs are bf16, sums fp32:
+    one bf16 rounding of the outputs, and the weight gradient in fp32 up to the order of its sums."""
+    from torsh_b200.ops.conv import conv2d_nhwc
+    torch.manual_seed(15)
+    x = torch.randn(n, hw, hw, ci, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    w = (torch.randn(co, ci, 3, 3, device=DEV) / (9 * ci) ** 0.5).to(torch.bfloat16).float().requires_grad_(True)
+    dy = torch.randn(n, hw, hw, co, device=DEV, dtype=torch.bfloat16)
+    y = conv2d_nhwc(x, w, 1, 1)
+    gx, gw = torch.autograd.grad(y, (x, w), dy)
+    xr, wr = x.detach().double().permute(0, 3, 1, 2).requires_grad_(True), w.detach().double().requires_grad_(True)
+    yr = torch.nn.functional.conv2d(xr, wr, padding=1)
+    rx, rw = torch.autograd.grad(yr, (xr, wr), dy.double().permute(0, 3, 1, 2))
+    assert _rel_elem(y, yr.permute(0, 2, 3, 1)) < 1e-2 and _rel_elem(gx, rx.permute(0, 2, 3, 1)) < 1e-2
+    assert _rel_elem(gw, rw) < 1e-3
+
+
+def test_conv1x1_fork_adds_the_skip_gradient():
+    from torsh_b200.ops.conv import conv1x1_fork_nhwc, conv2d_nhwc
+    torch.manual_seed(16)
+    x = torch.randn(3, 9, 10, 128, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    w = (torch.randn(64, 128, 1, 1, device=DEV) * 0.1).requires_grad_(True)
+    dy = torch.randn(3, 9, 10, 64, device=DEV, dtype=torch.bfloat16)
+    ds = torch.randn_like(x)
+    y, xx = conv1x1_fork_nhwc(x, w)
+    gx, gw = torch.autograd.grad((y, xx), (x, w), (dy, ds))
+    y0 = conv2d_nhwc(x, w)
+    g0, gw0 = torch.autograd.grad(y0, (x, w), dy)
+    assert torch.equal(y, y0) and _rel(gw, gw0) < 1e-5
+    assert _rel_elem(gx, g0.float() + ds.float()) < 1e-2
+    (only,) = torch.autograd.grad(conv1x1_fork_nhwc(x, w)[0].sum(), x)   # nothing flows back through the skip
+    assert _rel_elem(only, torch.autograd.grad(conv2d_nhwc(x, w).sum(), x)[0]) < 1e-2
+
+
 @pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1)])
 @pytest.mark.parametrize("shape", [(8, 64, 128), (16, 1024, 4096), (136, 200, 4160), (512, 1024, 4096), (264, 1608, 520)])
 def test_gemm_cluster_split_k(shape, majors):

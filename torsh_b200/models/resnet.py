@@ -110,8 +110,12 @@ class BottleneckBlock(nn.Module):
         return torch.relu(out + idt)
 
     def forward_nhwc(self, x):
+        if self.conv1.stride[0] == 1 and self.conv1.padding[0] == 0 and self.conv1.kernel_size == (1, 1):
+            out, x = cv.conv1x1_fork_nhwc(x, self.conv1.weight)
+        else:
+            out = _conv_nhwc(self.conv1, x)
         idt = x if self.downsample is None else _down_nhwc(self.downsample, x)
-        out = cv.batch_norm_nhwc(_conv_nhwc(self.conv1, x), self.bn1, relu=True)
+        out = cv.batch_norm_nhwc(out, self.bn1, relu=True)
         out = cv.batch_norm_nhwc(_conv_nhwc(self.conv2, out), self.bn2, relu=True)
         return cv.batch_norm_nhwc(_conv_nhwc(self.conv3, out), self.bn3, residual=idt, relu=True)
 

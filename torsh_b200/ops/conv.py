@@ -19,7 +19,7 @@ import os
 import torch
 
 from .. import _native as nv
-from ._dispatch import F, I, L, P, call, kernel_ok
+from ._dispatch import F, I, L, P, aligned, call, kernel_ok
 from .gemm import gemm
 
 
@@ -61,12 +61,17 @@ def _implicit_ok(c, co, kh, kw, stride, pad, w):
 
 
 def _wgrad_split(m_out, n_out, k):
+    """(tile width, K splits) of the weight gradient: the pixel dimension is cut so that the pieces fill whole waves of the
+    148 SMs, at least 16 K-blocks each; a piece costs its K-blocks plus about ten for filling and draining. (256 x 64 over
+    200 704 pixels: two tiles x 74 splits 26 us, x 98 splits 36 us.)"""
     bn = 256 if n_out >= 256 else 128
     tiles = ((m_out + 127) // 128) * ((n_out + bn - 1) // bn)
     kb = (k + 63) // 64
-    # measured on B200: the best split keeps tiles x splits within two waves of the 148 SMs and leaves every split
-    # at least 32 K-blocks (K = 8192: 32 tiles -> 4, 96 -> 3, 128 -> 2); deeper splits only add fp32 atomic traffic
-    return bn, max(1, min(296 // max(tiles, 1), kb // 32))
+
+    def cost(sk):
+        return -(-tiles * sk // 148) * (-(-kb // sk) + 10)
+    most = max(1, min(296 // max(tiles, 1), kb // 16))
+    return bn, min({max(1, min(most, w * 148 // tiles)) for w in (1, 2)} | {1}, key=cost)
 
 
 class _Conv2dFn(torch.autograd.Function):
@@ -108,7 +113,7 @@ class _Conv2dFn(torch.autograd.Function):
                     # dW = dy^T * shifted x, accumulated over pixel blocks straight from the two activations
                     kb = n * ((h + max(64 // w, 1) - 1) // max(64 // w, 1)) if h * w > 64 else (n + 64 // (h * w) - 1) // (64 // (h * w))
                     tiles = ((co + 127) // 128) * ((kpad + 255) // 256)
-                    sk = max(1, min(296 // max(tiles, 1), kb // 16))
+                    sk = max(1, min(296 // tiles, kb // 16))
                     g = torch.zeros(co, kpad, dtype=torch.float32, device=dy.device)
                     call("tb_conv3x3_wgrad", [P, P, P, I, I, I, I, I, I, I, I, P, P], dy2.data_ptr(), a.data_ptr(), g.data_ptr(),
                          n, h, w, c, co, kpad, sk, 0, nv.status_ptr(dy.device), nv.stream_ptr())
@@ -129,6 +134,43 @@ class _Conv2dFn(torch.autograd.Function):
             gemm(dy2, a, a_major=1, b_major=1, out=g, atomic=True, split_k=sk, bn=bn)   # dyᵀ · cols
             dw = g[:, :k].reshape(co, kh, kw, c).permute(0, 3, 1, 2).to(ctx.wdtype)
         return dx, dw, None, None
+
+
+class _Conv1x1ForkFn(torch.autograd.Function):
+    """``(conv1x1(x), x)``: the convolution and the untouched input as two outputs of one node, so that the backward adds the
+    gradient of the skip connection in the epilogue of the input-gradient GEMM instead of in a pass of its own."""
+
+    @staticmethod
+    def forward(ctx, x, weight):
+        return _Conv2dFn.forward(ctx, x, weight, 1, 0), x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dskip):
+        a, wm = ctx.saved_tensors
+        n, h, w, c, co = ctx.geom[:5]
+        dy2 = dy.reshape(n * h * w, co)
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        dx = dw = None
+        if ctx.needs_input_grad[0]:
+            res = None if dskip is None else aligned(dskip.reshape(n * h * w, c).to(dy2.dtype))
+            dx = gemm(dy2, wm, b_major=1, residual=res).view(n, h, w, c)
+        if ctx.needs_input_grad[1]:
+            bn, sk = _wgrad_split(co, c, dy2.shape[0])
+            g = torch.zeros(co, c, dtype=torch.float32, device=dy.device)
+            gemm(dy2, a, a_major=1, b_major=1, out=g, atomic=True, split_k=sk, bn=bn)
+            dw = g.reshape(ctx.wshape).to(ctx.wdtype)
+        return dx, dw
+
+
+def conv1x1_fork_nhwc(x: torch.Tensor, weight: torch.Tensor):
+    """``(conv2d_nhwc(x, weight), x)`` for a 1x1 / stride-1 convolution at the head of a residual block
+    (see :class:`_Conv1x1ForkFn`)."""
+    if (kernel_ok(x) and x.dtype == torch.bfloat16 and weight.shape[2:] == (1, 1) and weight.shape[0] % 8 == 0
+            and x.shape[-1] == weight.shape[1] and x.shape[-1] % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and x.requires_grad and torch.is_grad_enabled()):
+        return _Conv1x1ForkFn.apply(x, weight)
+    return conv2d_nhwc(x, weight), x
 
 
 def conv2d_nhwc(x: torch.Tensor, weight: torch.Tensor, stride: int = 1, padding: int = 0) -> torch.Tensor:
@@ -178,12 +220,12 @@ class _BatchNormFn(torch.autograd.Function):
         dy = dy.contiguous()
         dx = torch.empty_like(x)
         dres = torch.empty_like(x) if ctx.has_res else None
-        sums = torch.empty(2 * c, dtype=torch.float32, device=x.device)
-        dgb = torch.zeros(2, c, dtype=torch.float32, device=x.device)
+        sums = (torch.empty if rows else torch.zeros)(2 * c, dtype=torch.float32, device=x.device)
         call("tb_bn_bwd", [P, P, P, P, P, P, P, P, P, P, P, P, L, I, I, P], dy.data_ptr(), nv.ptr(y), x.data_ptr(),
              mean.data_ptr(), rstd.data_ptr(), g32.data_ptr(), b32.data_ptr(), sums.data_ptr(), dx.data_ptr(), nv.ptr(dres),
-             dgb[0].data_ptr(), dgb[1].data_ptr(), rows, c, int(ctx.relu), nv.stream_ptr())
-        return dx, dgb[0].to(ctx.pdtype), dgb[1].to(ctx.pdtype), dres, None, None, None, None, None
+             None, None, rows, c, int(ctx.relu), nv.stream_ptr())
+        # the column sums of the backward are the gradients of beta and gamma
+        return dx, sums[c:].to(ctx.pdtype), sums[:c].to(ctx.pdtype), dres, None, None, None, None, None
 
 
 def batch_norm_nhwc(x: torch.Tensor, bn: torch.nn.BatchNorm2d, residual: torch.Tensor | None = None,
