@@ -569,83 +569,47 @@ fa_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       for (int j = 0; j < n_kv; ++j, ++it) {
         const int kv0 = j * 128;
         const bool need_mask = (p.causal && kv0 + 127 > q0) || kv0 + 128 > p.S;
-        // With D = 64 the scores stay in registers and their columns are released at once. With D = 128 they are read again for
-        // the exponentials (their columns wait for P anyway), and the registers serve the rescaling of O in between.
-        constexpr int KEEP = ALIAS ? 2 : 4;
-        uint32_t v[KEEP][32];
+        uint32_t v[4][32];
         mbar_wait(s_full, it & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
         tc_fence_after();
-        float mx;
-        auto row_max = [&](const uint32_t (&x)[32], const uint32_t (&y)[32], int kv) {
-          return need_mask ? fa_row_max<true>(x, y, kv, col_limit) : fa_row_max<false>(x, y, kv, col_limit);
-        };
 #pragma unroll
-        for (int c = 0; c < KEEP; ++c) tmem_ld32(ts + c * 32, v[c]);
+        for (int c = 0; c < 4; ++c) tmem_ld32(ts + c * 32, v[c]);
         tmem_wait_ld();
-        if (ALIAS) {
-          mx = row_max(v[0], v[1], kv0);
-          tmem_ld32(ts + 64, v[0]);
-          tmem_ld32(ts + 96, v[1]);
-          tmem_wait_ld();
-          mx = fmaxf(mx, row_max(v[0], v[1], kv0 + 64));
-        } else {
+        if (!ALIAS) {
           tc_fence_before();
           mbar_arrive(s_free);
-          mx = fmaxf(row_max(v[0], v[1], kv0), row_max(v[KEEP - 2], v[KEEP - 1], kv0 + 64));
         }
+        const float mx = need_mask ? fmaxf(fa_row_max<true>(v[0], v[1], kv0, col_limit), fa_row_max<true>(v[2], v[3], kv0 + 64, col_limit))
+                                   : fmaxf(fa_row_max<false>(v[0], v[1], kv0, col_limit), fa_row_max<false>(v[2], v[3], kv0 + 64, col_limit));
+        const bool grow = mx > m;
+        const float mn = grow ? mx : m;
+        const float alpha = grow && j > 0 ? exp2f((m - mn) * sl2) : 1.f;
+        m = mn;
+        l2 = __fmul2_rn(l2, make_float2(alpha, alpha));
         if (it > 0) mbar_wait(pv_done, (it - 1) & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_EMPTY);  // P of block it - 1 is read
-        if (j == 0) {
-          m = mx;
-        } else {
-          const bool grow = mx > m;
-          if (__any_sync(0xffffffffu, grow)) {
-            const float mn = grow ? mx : m;
-            const float alpha = grow ? exp2f((m - mn) * sl2) : 1.f;
-            m = mn;
-            const float2 a2 = make_float2(alpha, alpha);
-            l2 = __fmul2_rn(l2, a2);
-            tc_fence_after();
-            constexpr int RC = ALIAS ? 4 : 1;   // 16-column pieces in registers at a time
-#pragma unroll 1
-            for (int c = 0; c < D; c += 16 * RC) {
-              uint32_t o[RC][16];
-#pragma unroll
-              for (int g = 0; g < RC; ++g) tmem_ld16(to + c + g * 16, o[g]);
-              tmem_wait_ld();
-#pragma unroll
-              for (int g = 0; g < RC; ++g) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) o[g][i] = __float_as_uint(__uint_as_float(o[g][i]) * alpha);
-                tmem_st16(to + c + g * 16, o[g]);
-              }
-            }
-            tmem_wait_st();
-          }
-        }
+        tc_fence_after();
         const float moff = (m == -INFINITY ? 0.f : m) * sl2;
-        uint32_t pk[4][16];
-        auto exps = [&](const uint32_t (&x)[32], int c) {
-          if (need_mask) fa_exp_pack<true>(x, sl2, moff, kv0 + c * 32, col_limit, pk[ALIAS ? c : 0], l2);
-          else fa_exp_pack<false>(x, sl2, moff, kv0 + c * 32, col_limit, pk[ALIAS ? c : 0], l2);
-        };
-        if (ALIAS) {
-          // columns 64 and up are still in registers; P goes out once the lower ones have been read, too
-          exps(v[0], 2);
-          exps(v[1], 3);
-          tmem_ld32(ts, v[0]);
-          tmem_ld32(ts + 32, v[1]);
-          tmem_wait_ld();
-          tmem_st16(tp + 32, pk[2]);
-          tmem_st16(tp + 48, pk[3]);
-          exps(v[0], 0);
-          tmem_st16(tp, pk[0]);
-          exps(v[1], 1);
-          tmem_st16(tp + 16, pk[1]);
-        } else {
 #pragma unroll
-          for (int c = 0; c < KEEP; ++c) {
-            exps(v[c], c);
-            tmem_st16(tp + c * 16, pk[0]);
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+          if (need_mask) fa_exp_pack<true>(v[c], sl2, moff, kv0 + c * 32, col_limit, pk, l2);
+          else fa_exp_pack<false>(v[c], sl2, moff, kv0 + c * 32, col_limit, pk, l2);
+          tmem_st16(tp + c * 16, pk);
+        }
+        // O is rescaled last: the registers of the scores are free by then and 64 columns go at once
+        if (j > 0 && __any_sync(0xffffffffu, grow)) {
+#pragma unroll 1
+          for (int c = 0; c < D; c += 64) {
+            uint32_t o[4][16];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) tmem_ld16(to + c + g * 16, o[g]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[g][i] = __float_as_uint(__uint_as_float(o[g][i]) * alpha);
+              tmem_st16(to + c + g * 16, o[g]);
+            }
           }
         }
         tmem_wait_st();
