@@ -26,6 +26,10 @@ struct GemmArgs {
   const void* aux;
   int flags, split_k;
   int* status;
+  // sums of A over K (a_major = 1: the columns of the stored [K, M] matrix), CTA-pair kernel only: null, or M values that the
+  // launch adds to (fp32) or, with colsum_store, writes in bf16 (split_k 1)
+  void* colsum = nullptr;
+  int colsum_store = 0;
 };
 
 // True when the kernel can run this product (alignment, epilogue).

@@ -13,6 +13,10 @@
 //               accumulation (TMA reduce-add) and, loaded while the tile's MMAs still run, the residual or the
 //               pre-activation of the GELU backward. No thread touches global memory row by row.
 // TMEM: two accumulators of 256 columns, so the epilogue of one tile runs under the MMAs of the next.
+// Weight gradients (A = dy, stored [tokens, outputs]) can carry the bias gradient: four more warps per CTA add up the A tiles
+// of the first column of output tiles over K, reading them from the stage between the MMAs that used it and its release.
+// As a kernel of its own the sum read dy once more from memory: 16 us of the 8192 x 1024 x 4096 MLP's backward and 0.78 ms
+// of a GPT-2-medium step; with it here, 8192 x 4096 x 1024 50.1 + 9.1 -> 52.5 us, 8192 x 3072 x 1024 39.3 + 7.2 -> 40.5.
 //
 // Every wait is bounded (sm100.cuh); a CTA that gives up drains its loops, and its peer runs into its own limits.
 #include <stdlib.h>
@@ -38,7 +42,7 @@ constexpr int SLOT_BYTES = 32 * 128;    // one staged group: 32 rows x 64 bf16 o
 constexpr int EPI_OFF = STAGES * STAGE_BYTES;
 constexpr int BAR_OFF = EPI_OFF + EPI_WARPS * 2 * SLOT_BYTES;
 // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], aux_full[EPI_WARPS][2], tmem pointer, abort flag
-constexpr int NBARS = 2 * STAGES + 4 + 2 * EPI_WARPS;
+constexpr int NBARS = 3 * STAGES + 4 + 2 * EPI_WARPS;  // used[STAGES] last
 constexpr int ALLOC = BAR_OFF + NBARS * 8 + 16;
 static_assert(ALLOC <= 232448, "shared memory budget of one CTA exceeded");
 
@@ -46,6 +50,8 @@ struct Params {
   int M, N, flags, split_k, tiles_m, tiles_n, kb_total, kb_per_split;
   const __nv_bfloat16* bias;
   int* status;
+  void* colsum;
+  int colsum_store;
 };
 
 struct Maps {
@@ -129,8 +135,8 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 
-template <int A_MAJOR, int B_MAJOR>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+template <int A_MAJOR, int B_MAJOR, bool COLSUM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS + (COLSUM ? 128 : 0), 1)
 gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {  // the 128-byte swizzle needs this alignment; the same in both CTAs
@@ -142,8 +148,10 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
   uint64_t* tmem_full = empty + STAGES;
   uint64_t* tmem_empty = tmem_full + 2;           // used in the leader only
   uint64_t* aux_full = tmem_empty + 2;
-  uint32_t* tmem_ptr = (uint32_t*)(aux_full + 2 * EPI_WARPS);
+  uint64_t* used = aux_full + 2 * EPI_WARPS;      // COLSUM: the MMAs of a stage are done, its A tile may be summed
+  uint32_t* tmem_ptr = (uint32_t*)(used + STAGES);
   volatile int* abort_flag = (volatile int*)(tmem_ptr + 1);
+  __shared__ float colsum_ex[COLSUM ? 128 : 1];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -152,7 +160,8 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], COLSUM ? 4 : 1);
+      mbar_init(&used[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
@@ -233,7 +242,7 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
           for (int k = 0; k < BK / 16; ++k)
             umma_pair(d_tmem, desc_at(adesc, k * (A_MAJOR == 0 ? 32 : 2048)), desc_at(bdesc, k * (B_MAJOR == 0 ? 32 : 2048)), idesc,
                    (kb > kb0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(&empty[s]);
+          umma_commit_pair(COLSUM ? &used[s] : &empty[s]);
           if (++s == STAGES) {
             s = 0;
             phase ^= 1;
@@ -243,6 +252,82 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1;
+        }
+      }
+    }
+  } else if (COLSUM && warp >= 2 + EPI_WARPS) {
+    // ---------------------------------------------------------------- column sums of A
+    // Two warps per 64-column chunk, 32 rows of a stage each: lane l reads the 16-byte vector l % 8 of rows l / 8, l / 8 + 4, ...
+    // (vectors are xored with row % 8), all eight before the first is added. The stage waits for this, so it has to be quick:
+    // with one warp per chunk and 4-byte reads the kernel took 75 us instead of 50.
+    const int id = warp - 2 - EPI_WARPS, chunk = id >> 1, r0 = (id & 1) * 32 + (lane >> 3);
+    int s = 0;
+    uint32_t phase = 0;
+    int m_t, n_t, kb0, kb1;
+    for (int w = worker; decode(p, w, m_t, n_t, kb0, kb1); w += nworkers) {
+      float2 total[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) total[j] = make_float2(0.f, 0.f);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const bool ok = mbar_wait(&used[s], phase, abort_flag, p.status, TB_ERR_WAIT_FULL);
+        if (n_t == 0 && ok) {
+          const uint8_t* base = smem + s * STAGE_BYTES + chunk * (64 * BK * 2);
+          uint4 x[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int k = r0 + 4 * i;
+            x[i] = *reinterpret_cast<const uint4*>(base + k * 128 + (((lane & 7) ^ (k & 7)) << 4));
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[s]);   // everything this warp needs of the stage is in registers
+          float2 part[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) part[j] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[j] = __fadd2_rn(part[j], make_float2(bf16_lo(u[j]), bf16_hi(u[j])));
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) total[j] = __fadd2_rn(total[j], part[j]);
+        } else if (lane == 0) {
+          mbar_arrive(&empty[s]);
+        }
+        if (++s == STAGES) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      if (n_t != 0) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+          total[j].x += __shfl_xor_sync(0xffffffffu, total[j].x, o);
+          total[j].y += __shfl_xor_sync(0xffffffffu, total[j].y, o);
+        }
+      const int m = m_t * 256 + (int)rank * 128 + chunk * 64 + (lane & 7) * 8;   // M is a multiple of 8
+      if (p.colsum_store) {
+        float4* ex = reinterpret_cast<float4*>(colsum_ex + chunk * 64 + (lane & 7) * 8);
+        if ((id & 1) && lane < 8) {
+          ex[0] = make_float4(total[0].x, total[0].y, total[1].x, total[1].y);
+          ex[1] = make_float4(total[2].x, total[2].y, total[3].x, total[3].y);
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + chunk) : "memory");
+        if (!(id & 1) && lane < 8 && m < p.M) {
+          const float4 a = ex[0], c = ex[1];
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.colsum) + m) =
+              make_uint4(pack_bf16x2(total[0].x + a.x, total[0].y + a.y), pack_bf16x2(total[1].x + a.z, total[1].y + a.w),
+                         pack_bf16x2(total[2].x + c.x, total[2].y + c.y), pack_bf16x2(total[3].x + c.z, total[3].y + c.w));
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + chunk) : "memory");
+      } else if (lane < 8 && m < p.M) {
+        float* out = reinterpret_cast<float*>(p.colsum) + m;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          atomicAdd(out + 2 * j, total[j].x);
+          atomicAdd(out + 2 * j + 1, total[j].y);
         }
       }
     }
@@ -396,9 +481,9 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
   }
 }
 
-template <int A_MAJOR, int B_MAJOR>
+template <int A_MAJOR, int B_MAJOR, bool COLSUM = false>
 static int launch(const Maps& maps, const Params& p, cudaStream_t stream) {
-  auto kern = gemm_pair_kernel<A_MAJOR, B_MAJOR>;
+  auto kern = gemm_pair_kernel<A_MAJOR, B_MAJOR, COLSUM>;
   static bool configured = false;
   if (!configured) {
     TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ALLOC));
@@ -406,7 +491,7 @@ static int launch(const Maps& maps, const Params& p, cudaStream_t stream) {
   }
   const long total = (long)p.tiles_m * p.tiles_n * p.split_k;
   const int pairs = sm_count() / 2;
-  kern<<<2 * (int)(total < pairs ? total : pairs), THREADS, ALLOC, stream>>>(maps, p);
+  kern<<<2 * (int)(total < pairs ? total : pairs), THREADS + (COLSUM ? 128 : 0), ALLOC, stream>>>(maps, p);
   TB_CUDA_CHECK(cudaGetLastError());
   return TB_LAUNCH_OK;
 }
@@ -470,6 +555,13 @@ int gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
   if (a.flags & EPI_RESIDUAL) {
     str[0] = (uint64_t)a.ldr * 2;
     if ((r = make_tmap(&m.aux, a.residual, 2, 2, dims, str, box))) return r;
+  }
+  if (a.colsum) {
+    if (a.a_major != 1 || a.b_major != 1 || (a.colsum_store && p.split_k > 1) || ((uintptr_t)a.colsum & 15) || a.M % 8)
+      TB_FAIL(TB_E_ARG, "gemm_pair: column sums need MN-major operands, M a multiple of 8, 16-byte alignment and, to be written, no split");
+    p.colsum = a.colsum;
+    p.colsum_store = a.colsum_store;
+    return launch<1, 1, true>(m, p, stream);
   }
   if (a.a_major == 0) return a.b_major == 0 ? launch<0, 0>(m, p, stream) : launch<0, 1>(m, p, stream);
   return a.b_major == 0 ? launch<1, 0>(m, p, stream) : launch<1, 1>(m, p, stream);

@@ -1069,6 +1069,20 @@ TB_EXPORT int tb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, 
                        split_k, bn, status, stream, TpFusion{});
 }
 
+// Weight gradient with the bias gradient: D[M, N] (+)= A^T B for A = dy [K, M], B = x [K, N] (bf16), and colsum[M] = the sums of
+// A over K. accumulate: D is fp32 and added to, colsum fp32 and added to (split_k >= 1); else D and colsum are bf16 and written.
+TB_EXPORT int tb_gemm_wgrad(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, void* colsum,
+                            int accumulate, int split_k, int* status, cudaStream_t stream) {
+  TB_ENSURE_DEVICE();
+  if (!A || !B || !D || !colsum || M <= 0 || N <= 0 || K <= 0 || (lda & 7) || (ldb & 7) || (!accumulate && split_k > 1))
+    TB_FAIL(TB_E_ARG, "gemm_wgrad: null pointer, empty shape, lda / ldb not multiples of 8, or a split without accumulation");
+  GemmArgs ga{A, B, D, M, N, K, 1, 1, lda, ldb, ldd, nullptr, nullptr, 0, nullptr, nullptr,
+              accumulate ? EPI_OUT_F32 | EPI_ATOMIC : 0, split_k, status};
+  ga.colsum = colsum;
+  ga.colsum_store = !accumulate;
+  return gemm_pair_launch(ga, stream);
+}
+
 // 3x3 / stride 1 / pad 1 convolution as an implicit GEMM (no im2col buffer). x: channels-last bf16 [n, h, w, c] with
 // c % 64 == 0 and w <= 128. mode 1 (forward): wmat = [cout, 9*c] (taps row-major, channels innermost), y = [n*h*w, cout].
 // mode 2 (input gradient): x is the output gradient [n, h, w, cout_fwd] (so c = cout_fwd), wmat is the SAME forward

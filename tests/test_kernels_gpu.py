@@ -145,6 +145,29 @@ def test_gemm_pair_tiles_and_epilogues(shape, majors):
     nv.check_status()
 
 
+@pytest.mark.parametrize("tokens,m,n", [(1, 256, 256), (77, 264, 520), (1000, 4096, 1024), (333, 2568, 1288), (8192, 1024, 1024), (65, 9472, 256)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_weight_gradient_carries_the_bias_gradient(tokens, m, n, accumulate):
+    """Both destinations (fresh bf16 gradients, fp32 buffers that are added to, with K split where the plan splits it), ragged
+    tiles and remainders of tokens. Fresh gradients carry one bf16 rounding; fp32 sums of at most 8192 bf16 values differ by
+    their order: about 2^-24 * sqrt(8192) of their rms, far below 1e-4."""
+    from torsh_b200.ops.linear import linear
+    torch.manual_seed(17)
+    x = torch.randn(tokens, n, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(m, n, device=DEV) * 0.02).to(torch.bfloat16).requires_grad_(True)
+    b = torch.randn(m, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    dy = torch.randn(tokens, m, device=DEV, dtype=torch.bfloat16)
+    rw, rb = dy.double().t() @ x.double(), dy.double().sum(0)
+    if accumulate:
+        w.main_grad, b.main_grad = torch.ones(m, n, device=DEV), torch.ones(m, device=DEV)
+    gw, gb = torch.autograd.grad(linear(x, w, b), (w, b), dy, allow_unused=True)
+    if accumulate:
+        assert gw is None and gb is None
+        assert _rel_elem(w.main_grad, rw + 1) < 1e-4 and _rel_elem(b.main_grad, rb + 1) < 1e-4
+    else:
+        assert _rel_elem(gw, rw) < 1e-2 and _rel_elem(gb, rb) < 1e-2
+
+
 @pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
 @pytest.mark.parametrize("shape", [(40000, 64, 256), (39992, 8, 64), (30000, 56, 72)])
 def test_gemm_narrow_outputs(shape, majors):

@@ -14,6 +14,7 @@ import os
 import torch
 
 from .. import _native as nv
+from ._dispatch import call
 
 EPI_BIAS = 1
 EPI_GELU = 2
@@ -154,3 +155,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
         nv.check(rc, "tb_gemm_bf16")
     nv.launch_count += 1
     return out
+
+
+_WGRAD = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 6 + [ctypes.c_void_p] + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2
+
+
+def gemm_wgrad_bias(dy: torch.Tensor, x: torch.Tensor, dw: torch.Tensor, db: torch.Tensor, accumulate: bool,
+                    split_k: int = 1) -> None:
+    """``dw = dyᵀ x`` and ``db = Σ rows of dy`` in one launch, on CTA pairs. ``accumulate``: both fp32 and added to; otherwise both
+    bf16 and written (no split)."""
+    k, m = dy.shape
+    call("tb_gemm_wgrad", _WGRAD, dy.data_ptr(), x.data_ptr(), dw.data_ptr(), m, x.shape[1], k, dy.stride(0), x.stride(0),
+         dw.stride(0), db.data_ptr(), int(accumulate), split_k, nv.status_ptr(dy.device), nv.stream_ptr())

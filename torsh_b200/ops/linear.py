@@ -14,7 +14,7 @@ import torch
 
 from . import elementwise as ew
 from ._dispatch import kernel_ok
-from .gemm import gemm
+from .gemm import gemm, gemm_wgrad_bias
 
 
 # TORSH_WGRAD_STREAM_K=0 goes back to uniform K-splits for the weight-gradient GEMMs
@@ -87,6 +87,30 @@ def _bgrad(dy2: torch.Tensor, bias: torch.Tensor):
     return g.to(bias.dtype)
 
 
+def _wgrad_bgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layout: str, bias, need_w: bool, need_b: bool):
+    """Gradients of weight and bias. Where the weight gradient runs on CTA pairs it carries the bias gradient (same kind of
+    destination for both, [out, in] weights): ``dy`` is then not read a second time."""
+    need_b = need_b and bias is not None
+    if need_w and need_b and layout == "nk":
+        m, n, k = dy2.shape[1], x2.shape[1], dy2.shape[0]
+        wmg, bmg = getattr(weight, "main_grad", None), getattr(bias, "main_grad", None)
+        tiles = ((m + 255) // 256) * ((n + 255) // 256)
+        if m >= 256 and n >= 256 and m % 8 == 0 and n % 8 == 0 and dy2.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0:
+            if wmg is not None and bmg is not None:
+                if wmg.is_contiguous() and bmg.is_contiguous() and wmg.data_ptr() % 16 == 0 and bmg.data_ptr() % 16 == 0:
+                    gemm_wgrad_bias(dy2, x2, wmg, bmg, True, _wgrad_pair_split(m, n, k, True))
+                    return None, None
+            # without a buffer to accumulate into: only where no split is wanted and the tiles fill half of the 74 pairs
+            elif (wmg is None and bmg is None and tiles >= 37 and weight.dtype == bias.dtype == torch.bfloat16
+                  and _wgrad_pair_split(m, n, k, False) == 1):
+                dw = torch.empty(m, n, dtype=torch.bfloat16, device=dy2.device)
+                db = torch.empty(m, dtype=torch.bfloat16, device=dy2.device)
+                gemm_wgrad_bias(dy2, x2, dw, db, False)
+                return dw, db.view(bias.shape)
+    dw = _wgrad(dy2, x2, weight, layout) if need_w else None
+    return dw, (_bgrad(dy2, bias) if need_b else None)
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, layout, gelu, residual):
@@ -115,8 +139,7 @@ class _LinearFn(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, weight, b_major=1 if layout == "nk" else 0).view(ctx.xshape)
-        dw = _wgrad(dy2, x2, weight, layout) if ctx.needs_input_grad[1] else None
-        db = _bgrad(dy2, bias) if bias is not None and ctx.needs_input_grad[2] else None
+        dw, db = _wgrad_bgrad(dy2, x2, weight, layout, bias, ctx.needs_input_grad[1], ctx.needs_input_grad[2])
         return dx, dw, db, None, None, dres
 
 
@@ -141,13 +164,14 @@ class _MlpFn(torch.autograd.Function):
     """``y = gelu(x W1ᵀ + b1) W2ᵀ + b2 + residual`` with the GELU derivative fused into the fc2 dgrad epilogue."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, residual):
+    def forward(ctx, x, w1, b1, w2, b2, residual, keep):
         K = x.shape[-1]
         x2 = x.reshape(-1, K)
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         M, Fh = x2.shape[0], w1.shape[0]
-        u = torch.empty(M, Fh, dtype=x.dtype, device=x.device)
+        # the pre-activation is written only for a backward pass
+        u = torch.empty(M, Fh, dtype=x.dtype, device=x.device) if keep else None
         h = gemm(x2, w1, bias=b1, gelu=True, preact_out=u)
         res2 = residual.reshape(M, -1) if residual is not None else None
         y = gemm(h, w2, bias=b2, residual=res2)
@@ -162,18 +186,17 @@ class _MlpFn(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         du = gemm(dy2, w2, b_major=1, dgelu_aux=u)          # (dy W2) * gelu'(u)
-        dw2 = _wgrad(dy2, h, w2, "nk")
-        db2 = _bgrad(dy2, ctx.b2) if ctx.b2 is not None else None
+        dw2, db2 = _wgrad_bgrad(dy2, h, w2, "nk", ctx.b2, True, True)
         dx = gemm(du, w1, b_major=1).view(ctx.xshape) if ctx.needs_input_grad[0] else None
-        dw1 = _wgrad(du, x2, w1, "nk")
-        db1 = _bgrad(du, ctx.b1) if ctx.b1 is not None else None
-        return dx, dw1, db1, dw2, db2, (dy if ctx.has_res else None)
+        dw1, db1 = _wgrad_bgrad(du, x2, w1, "nk", ctx.b1, True, True)
+        return dx, dw1, db1, dw2, db2, (dy if ctx.has_res else None), None
 
 
 def mlp_gelu(x, w1, b1, w2, b2, residual=None):
     """Transformer MLP block (weights in ``[out, in]`` layout) with optional fused residual add."""
     if kernel_ok(x, w1, b1, w2, b2, residual) and x.dtype == torch.bfloat16 and w1.dtype == torch.bfloat16:
-        return _MlpFn.apply(x, w1, b1, w2, b2, residual)
+        keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, w1, b1, w2, b2, residual))
+        return _MlpFn.apply(x, w1, b1, w2, b2, residual, keep)
     h = torch.nn.functional.gelu(torch.nn.functional.linear(x, w1.to(x.dtype), b1), approximate="tanh")
     y = torch.nn.functional.linear(h, w2.to(x.dtype), b2)
     return y if residual is None else y + residual
