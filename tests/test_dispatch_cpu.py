@@ -1,0 +1,56 @@
+"""Rules that pick a kernel or refuse a call, without a GPU: the launching functions are replaced by recorders."""
+import pytest
+import torch
+
+
+@pytest.fixture
+def wgrad_calls(monkeypatch):
+    """Names of the launching functions that the gradients of a linear layer reach, in order."""
+    from torsh_b200.ops import linear as L
+    calls = []
+    monkeypatch.setattr(L, "gemm_wgrad_bias", lambda *a, **k: calls.append("wgrad_bias"))
+    monkeypatch.setattr(L, "gemm", lambda a, b, **k: calls.append("gemm") or k.get("out"))
+    monkeypatch.setattr(L.ew, "colsum_into", lambda *a: calls.append("colsum"))
+    return calls
+
+
+def _layer(wmg, bmg, m=512, n=256):
+    w, b = torch.zeros(m, n, dtype=torch.bfloat16), torch.zeros(m, dtype=torch.bfloat16)
+    w.main_grad, b.main_grad = wmg, bmg
+    return torch.zeros(64, m, dtype=torch.bfloat16), torch.zeros(64, n, dtype=torch.bfloat16), w, b
+
+
+@pytest.mark.parametrize("wmg,bmg,carried", [
+    (torch.zeros(512, 256), torch.zeros(512), True),
+    (torch.zeros(512, 256, dtype=torch.bfloat16), torch.zeros(512), False),
+    (torch.zeros(512, 256), torch.zeros(512, dtype=torch.bfloat16), False),
+    (torch.zeros(256, 512), torch.zeros(512), False),
+    (torch.zeros(511, 256), torch.zeros(512), False),
+    (torch.zeros(512, 256), torch.zeros(256), False),
+    (torch.zeros(512, 512)[:, ::2], torch.zeros(512), False),
+])
+def test_bias_gradient_rides_only_into_fp32_buffers_of_the_right_shape(wgrad_calls, wmg, bmg, carried):
+    """The fused launch adds through raw pointers: a buffer that it would overrun goes to the ops that check theirs."""
+    from torsh_b200.ops.linear import _wgrad_bgrad
+    dy, x, w, b = _layer(wmg, bmg)
+    assert _wgrad_bgrad(dy, x, w, "nk", b, True, True) == (None, None)
+    assert wgrad_calls == (["wgrad_bias"] if carried else ["gemm", "colsum"])
+
+
+def test_column_sums_refuse_other_buffers(monkeypatch):
+    """The kernel adds fp32 values through the buffer's pointer; without the kernel any buffer that add_ takes is fine."""
+    from torsh_b200.ops import elementwise as ew
+    x, other = torch.ones(4, 8), (torch.zeros(8, dtype=torch.bfloat16), torch.zeros(7), torch.zeros(16)[::2])
+    out = torch.zeros(8, dtype=torch.bfloat16)
+    ew.colsum_into(x, out)
+    assert (out == 4).all()
+    calls = []
+    monkeypatch.setattr(ew, "kernel_ok", lambda *t: True)
+    monkeypatch.setattr(ew, "call", lambda name, *a: calls.append(name))
+    monkeypatch.setattr(ew.nv, "stream_ptr", lambda *a: None)
+    for bad in other:
+        with pytest.raises(AssertionError):
+            ew.colsum_into(x, bad)
+    assert calls == []
+    ew.colsum_into(x, torch.zeros(8))
+    assert calls == ["tb_colsum"]

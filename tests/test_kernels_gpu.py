@@ -168,6 +168,22 @@ def test_weight_gradient_carries_the_bias_gradient(tokens, m, n, accumulate):
         assert _rel_elem(gw, rw) < 1e-2 and _rel_elem(gb, rb) < 1e-2
 
 
+@pytest.mark.parametrize("wmg,bmg", [((torch.bfloat16, (512, 256)), (torch.float32, (512,))), ((torch.float32, (256, 512)), (torch.float32, (512,))),
+                                     ((torch.float32, (512, 256)), (torch.bfloat16, (512,))), ((torch.float32, (512, 256)), (torch.float32, (256,)))])
+def test_gradient_buffers_of_another_kind_are_refused(wmg, bmg):
+    from torsh_b200 import _native as nv
+    from torsh_b200.ops.gemm import gemm_wgrad_bias
+    from torsh_b200.ops.linear import linear
+    x, dy = torch.randn(64, 256, device=DEV, dtype=torch.bfloat16), torch.randn(64, 512, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(512, 256, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    b = torch.randn(512, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    w.main_grad, b.main_grad = (torch.zeros(s, device=DEV, dtype=d) for d, s in (wmg, bmg))
+    with pytest.raises((AssertionError, nv.NativeError)):
+        torch.autograd.grad(linear(x, w, b), (w, b), dy, allow_unused=True)
+    with pytest.raises(AssertionError):
+        gemm_wgrad_bias(dy, x, w.main_grad, b.main_grad, True)
+
+
 @pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
 @pytest.mark.parametrize("shape", [(40000, 64, 256), (39992, 8, 64), (30000, 56, 72)])
 def test_gemm_narrow_outputs(shape, majors):

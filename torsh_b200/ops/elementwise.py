@@ -256,6 +256,8 @@ def rope(x: torch.Tensor, base: float = 10000.0, pos_offset: int = 0) -> torch.T
 def colsum_into(x2d: torch.Tensor, out_f32: torch.Tensor) -> None:
     """``out_f32[c] += Σ_r x2d[r, c]`` (bias gradients; fp32 accumulation)."""
     if kernel_ok(x2d) and x2d.stride(1) == 1:
+        assert out_f32.dtype == torch.float32 and out_f32.numel() == x2d.shape[1] and out_f32.is_contiguous()
+        assert out_f32.device == x2d.device
         call("tb_colsum", [P, P, L, I, L, I, P], x2d.data_ptr(), out_f32.data_ptr(), x2d.shape[0], x2d.shape[1],
              x2d.stride(0), dtype_code(x2d), nv.stream_ptr())
     else:

@@ -164,6 +164,11 @@ def gemm_wgrad_bias(dy: torch.Tensor, x: torch.Tensor, dw: torch.Tensor, db: tor
                     split_k: int = 1) -> None:
     """``dw = dyᵀ x`` and ``db = Σ rows of dy`` in one launch, on CTA pairs. ``accumulate``: both fp32 and added to; otherwise both
     bf16 and written (no split)."""
-    k, m = dy.shape
-    call("tb_gemm_wgrad", _WGRAD, dy.data_ptr(), x.data_ptr(), dw.data_ptr(), m, x.shape[1], k, dy.stride(0), x.stride(0),
+    assert dy.dtype == x.dtype == torch.bfloat16 and dy.dim() == x.dim() == 2 and dy.stride(1) == x.stride(1) == 1
+    (k, m), n = dy.shape, x.shape[1]
+    assert x.shape[0] == k, f"contraction mismatch {k} vs {x.shape[0]}"
+    assert dw.shape == (m, n) and dw.stride(1) == 1 and db.numel() == m and db.is_contiguous()
+    assert dw.dtype == db.dtype == (torch.float32 if accumulate else torch.bfloat16)
+    assert x.device == dw.device == db.device == dy.device and dy.is_cuda
+    call("tb_gemm_wgrad", _WGRAD, dy.data_ptr(), x.data_ptr(), dw.data_ptr(), m, n, k, dy.stride(0), x.stride(0),
          dw.stride(0), db.data_ptr(), int(accumulate), split_k, nv.status_ptr(dy.device), nv.stream_ptr())

@@ -87,6 +87,12 @@ def _bgrad(dy2: torch.Tensor, bias: torch.Tensor):
     return g.to(bias.dtype)
 
 
+def _adds_in_place(buf: torch.Tensor, shape: tuple, device) -> bool:
+    """A ``main_grad`` that a kernel may add to through its pointer: anything else goes to the ops that refuse it."""
+    return (buf.dtype == torch.float32 and buf.shape == shape and buf.is_contiguous() and buf.data_ptr() % 16 == 0
+            and buf.device == device)
+
+
 def _wgrad_bgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layout: str, bias, need_w: bool, need_b: bool):
     """Gradients of weight and bias. Where the weight gradient runs on CTA pairs it carries the bias gradient (same kind of
     destination for both, [out, in] weights): ``dy`` is then not read a second time."""
@@ -97,7 +103,7 @@ def _wgrad_bgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layo
         tiles = ((m + 255) // 256) * ((n + 255) // 256)
         if m >= 256 and n >= 256 and m % 8 == 0 and n % 8 == 0 and dy2.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0:
             if wmg is not None and bmg is not None:
-                if wmg.is_contiguous() and bmg.is_contiguous() and wmg.data_ptr() % 16 == 0 and bmg.data_ptr() % 16 == 0:
+                if _adds_in_place(wmg, (m, n), dy2.device) and _adds_in_place(bmg, (m,), dy2.device):
                     gemm_wgrad_bias(dy2, x2, wmg, bmg, True, _wgrad_pair_split(m, n, k, True))
                     return None, None
             # without a buffer to accumulate into: only where no split is wanted and the tiles fill half of the 74 pairs
