@@ -450,6 +450,57 @@ def test_cross_entropy_row_sizes(dtype, V, ld, rows):
     assert abs(neg.item() + 2 * torch.nn.functional.cross_entropy(ref_in.detach(), tg.clamp(min=0)).item()) < 1e-3 * max(1.0, abs(neg.item()))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [9, 1003, 4096, 20011, 60001])
+def test_cross_entropy_in_place_reads_its_target_first(dtype, V):
+    """The gradient overwrites the logits while other threads still work on the row: a target in the first, in the last and in
+    scattered vectors, several rows a CTA. A target's own logit is far from the others, so the mean shows a single wrong one:
+    the gap is 20 in 2000 rows, against a mean that fp32 sums in another order move by less than 1e-3."""
+    from torsh_b200.ops.softmax import cross_entropy
+    torch.manual_seed(10)
+    rows = 2000
+    tg = torch.randint(0, V, (rows,), device=DEV)
+    tg[:4] = torch.tensor([0, V - 1, V // 2, V - V % 8 - 1], device=DEV)
+    x = torch.randn(rows, (V + 7) // 8 * 8, device=DEV)
+    x[torch.arange(rows, device=DEV), tg] = -20.0
+    x = x.to(dtype)
+    ref = torch.nn.functional.cross_entropy(x[:, :V].double(), tg)
+    y = x.clone().requires_grad_(True) * 1.0
+    loss = cross_entropy(y, tg, num_classes=V, inplace_grad=True, root_scale=1.0)
+    assert abs(loss.item() - ref.item()) < 1e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [40, 1000, 20011])
+def test_cross_entropy_masked_logits(dtype, V):
+    """Columns masked with -inf or with the type's lowest value, whole vectors and single columns of them; a row that is masked
+    throughout, one with a NaN and one with +inf give what log_softmax gives, and leave the other rows alone."""
+    from torsh_b200.ops.softmax import cross_entropy
+    torch.manual_seed(18)
+    rows, low = 24, torch.finfo(dtype).min
+    x = torch.randn(rows, (V + 7) // 8 * 8, device=DEV).to(dtype)
+    x[:6, ::3] = float("-inf")
+    x[6:12, 8:V - 8] = low
+    x[12:18, 1:] = float("-inf")
+    tg = torch.full((rows,), 1, device=DEV)
+    tg[12:18] = 0
+    x[18], x[19, 5], x[20, 7], x[21] = float("-inf"), float("nan"), float("inf"), low
+    ref_in = x[:, :V].double().requires_grad_(True)
+    row_loss = torch.nn.functional.cross_entropy(ref_in, tg, reduction="none")
+    row_loss[[r for r in range(rows) if r not in (18, 19, 20)]].sum().backward()
+    fine = [r for r in range(rows) if r not in (18, 19, 20, 21)]
+    for r in range(rows):
+        one = cross_entropy(x[r:r + 1].contiguous(), tg[r:r + 1], num_classes=V).double()
+        if r in (18, 19, 20):
+            assert not torch.isfinite(one) and not torch.isfinite(row_loss[r])
+        elif r != 21:   # in fp32 the lowest value absorbs log(V)
+            assert abs(one.item() - row_loss[r].item()) < 1e-4 * max(1.0, abs(row_loss[r].item()))
+    lg = x.clone().requires_grad_(True)
+    (g,) = torch.autograd.grad(cross_entropy(lg, tg, num_classes=V, root_scale=float(rows)), lg)
+    assert _rel(g[fine, :V], ref_in.grad[fine]) < (1e-2 if dtype == torch.bfloat16 else 1e-4)
+    assert g[:, V:].abs().sum().item() == 0.0
+
+
 # ------------------------------------------------------------------ elementwise / reduce / embedding / rope
 def test_unary_binary_reduce():
     from torsh_b200.ops import elementwise as ew
