@@ -36,7 +36,8 @@ constexpr int FB_THREADS = 512;
 struct FaBwdParams {
   const float* LSE;    // [B, H, S]
   const float* delta;  // [B, H, S]  rowsum(dO * O)
-  float* dQ_acc;       // fp32, accumulated: [B*H][query blocks][D / 32][128 rows][32 columns, 16-byte chunks xor row % 8]
+  float* dQ_acc;       // fp32, accumulated: [B*H][groups of 32 queries][D / 32][the group's rows][32 columns, 16-byte chunks
+                       // xor row % 8]; the last group of a sequence has S % 32 rows, so this is B*H*S*D floats
   __nv_bfloat16* dK;   // [B*S, dkv_stride], head h at column h*D
   __nv_bfloat16* dV;
   int B, S, H;
@@ -328,7 +329,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     for (int t = 0; t < n_it; ++t) {
       mbar_wait(dq_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
-      float* dq_blk = p.dQ_acc + (((size_t)bh * n_blk + i0 + t) * (D / 32)) * 4096 + (warp & 3) * 1024;
+      const int row0 = (i0 + t) * 128 + (warp & 3) * 32, rows = min(32, p.S - row0);
+      if (rows <= 0) {   // nothing of this warp's quarter is in the sequence
+        tc_fence_before();
+        mbar_arrive(dq_empty);
+        continue;
+      }
+      float* dq_grp = p.dQ_acc + ((size_t)bh * p.S + row0) * D;
 #pragma unroll
       for (int c = 0; c < D / 32; c += 2) {
         // both columns groups to registers first: with the last pair the columns are free before anything is staged
@@ -353,8 +360,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         if (lane == 0) {
 #pragma unroll
           for (int k = 0; k < 2; ++k)
-            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_blk + (c + k) * 4096),
-                         "r"(smem_u32(stage + k * 4096)), "r"(4096)
+            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_grp + (c + k) * rows * 32),
+                         "r"(smem_u32(stage + k * 4096)), "r"(rows * 128)
                          : "memory");
           bulk_commit();
         }
@@ -485,9 +492,9 @@ __global__ void fa_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_
   }
 }
 
-// dQ: the fp32 accumulator's blocks (layout at FaBwdParams::dQ_acc) -> bf16 rows. One thread per 8 columns of a row.
+// dQ: the fp32 accumulator's groups (layout at FaBwdParams::dQ_acc) -> bf16 rows. One thread per 8 columns of a row.
 __global__ void fa_cvt_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int B, int S, int H, int D,
-                                 int n_blk, long dst_stride) {
+                                 long dst_stride) {
   const int vpr = D / 8;  // vectors per (token, head)
   const long total = (long)B * S * H * vpr;
   const long stride = (long)gridDim.x * blockDim.x;
@@ -497,8 +504,8 @@ __global__ void fa_cvt_dq_kernel(const float* __restrict__ src, __nv_bfloat16* _
     const int h = (int)(th % H);
     const long tok = th / H;
     const int b = (int)(tok / S), s = (int)(tok - (long)b * S);
-    const int row = s & 127, c = v >> 2, g = (v & 3) * 2;
-    const float* blk = src + ((((size_t)b * H + h) * n_blk + (s >> 7)) * (D / 32) + c) * 4096 + row * 32;
+    const int row = s & 31, c = v >> 2, g = (v & 3) * 2, rows = min(32, S - (s - row));
+    const float* blk = src + (((size_t)b * H + h) * S + (s - row)) * D + (c * rows + row) * 32;
     const float4 x = *reinterpret_cast<const float4*>(blk + ((g ^ (row & 7)) << 2));
     const float4 y = *reinterpret_cast<const float4*>(blk + (((g + 1) ^ (row & 7)) << 2));
     *reinterpret_cast<uint4*>(dst + tok * dst_stride + (long)h * D + v * 8) =
@@ -516,7 +523,7 @@ inline int make_bshd_map_bwd(CUtensorMap* m, const void* base, int B, int S, int
 }  // namespace tb
 using namespace tb;
 
-// Workspace (caller-provided, 16-byte aligned): delta fp32 [B*H*S], dq_acc fp32 [B*H*ceil(S/128)*128*D] (zeroed here).
+// Workspace (caller-provided, 16-byte aligned): delta fp32 [B*H*S], dq_acc fp32 [B*S*H*D] (zeroed here).
 // dq, dk, dv: bf16 [B*S, dqkv_stride] with head h at column h*D (may be the three column bands of
 // one fused dQKV buffer).
 TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
@@ -543,7 +550,7 @@ TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, con
     fa_delta_kernel<64><<<(unsigned)((nthreads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_stride, do_stride);
   else
     fa_delta_kernel<128><<<(unsigned)((nthreads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_stride, do_stride);
-  TB_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * H * ((S + 127) / 128) * 128 * D, st));
+  TB_CUDA_CHECK(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * S * H * D, st));
   FaBwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, B, S, H, dqkv_stride, scale, causal, status};
   const int n_blk = (S + 127) / 128;
   const long grid = (long)n_blk * B * H;
@@ -558,7 +565,7 @@ TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, con
   }
   const long items = (long)B * S * H * (D / 8);
   int g = (int)((items + 255) / 256 < (long)sm_count() * 16 ? (items + 255) / 256 : (long)sm_count() * 16);
-  fa_cvt_dq_kernel<<<g, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, B, S, H, D, n_blk, dqkv_stride);
+  fa_cvt_dq_kernel<<<g, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dq, B, S, H, D, dqkv_stride);
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -25,7 +25,7 @@ def _fwd(q, k, v, out, lse, B, S, H, D, q_stride, kv_stride, scale, causal):
 
 def _bwd(q, k, v, o, do, lse, dq, dk, dv, B, S, H, D, q_stride, kv_stride, dqkv_stride, scale, causal):
     delta = torch.empty(B * H * S, dtype=torch.float32, device=q.device)
-    dq_acc = torch.empty(B * H * ((S + 127) // 128 * 128) * D, dtype=torch.float32, device=q.device)
+    dq_acc = torch.empty(B * S * H * D, dtype=torch.float32, device=q.device)
     call("tb_flash_attn_bwd", _BWD, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(),
          lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), B, S, H, D,
          q_stride, kv_stride, o.stride(0), do.stride(0), dqkv_stride, float(scale), int(causal),
