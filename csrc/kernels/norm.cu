@@ -448,41 +448,45 @@ __global__ void __launch_bounds__(NW * 32, 1) norm_bwd_ring_kernel(
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // the teams take turns adding their column sums into [2][H] floats over the ring's memory
+  // every team with a row leaves its column sums in its own [2][H] floats (RMS: [H]) over the ring's memory, which they never
+  // exceed, and the CTA adds them in the order of the teams. Taking turns at one [2][H], 8 to 24 barriers, was most of a call
+  // with few rows.
   float* sums = reinterpret_cast<float*>(nb_smem);
-  for (int t = 0; t < teams; ++t) {
-    if (active && team == t) {
+  const int width = RMS ? H : 2 * H, filled = min(teams, rows - (int)blockIdx.x * teams);
+  if (active && team < filled) {
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int v = member * 32 + lane + i * 32 * G;
-        if (v < nvec) {
+    for (int i = 0; i < VPL; ++i) {
+      const int v = member * 32 + lane + i * 32 * G;
+      if (v < nvec) {
 #pragma unroll
-          for (int j = 0; j < N; j += 4) {
-            float4* pg = reinterpret_cast<float4*>(sums + v * N + j);
-            float4* pb = reinterpret_cast<float4*>(sums + H + v * N + j);
-            float4 a = make_float4(dg[i][j / 2].x, dg[i][j / 2].y, dg[i][j / 2 + 1].x, dg[i][j / 2 + 1].y);
-            float4 c = make_float4(db[i][j / 2].x, db[i][j / 2].y, db[i][j / 2 + 1].x, db[i][j / 2 + 1].y);
-            if (t > 0) {
-              const float4 a0 = *pg, c0 = *pb;
-              a.x += a0.x; a.y += a0.y; a.z += a0.z; a.w += a0.w;
-              c.x += c0.x; c.y += c0.y; c.z += c0.z; c.w += c0.w;
-            }
-            *pg = a;
-            if (!RMS) *pb = c;
-            else if (t == 0) *pb = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
+        for (int j = 0; j < N; j += 4) {
+          float* at = sums + (size_t)team * width + v * N + j;
+          *reinterpret_cast<float4*>(at) = make_float4(dg[i][j / 2].x, dg[i][j / 2].y, dg[i][j / 2 + 1].x, dg[i][j / 2 + 1].y);
+          if (!RMS)
+            *reinterpret_cast<float4*>(at + H) = make_float4(db[i][j / 2].x, db[i][j / 2].y, db[i][j / 2 + 1].x, db[i][j / 2 + 1].y);
         }
       }
     }
-    __syncthreads();
   }
-  for (int c = threadIdx.x; c < H; c += blockDim.x) {
-    if (partial) {
-      partial[(size_t)blockIdx.x * 2 * H + c] = sums[c];
-      if (!RMS) partial[(size_t)blockIdx.x * 2 * H + H + c] = sums[H + c];
-    } else {
-      if (dgamma) atomicAdd(dgamma + c, sums[c]);
-      if (!RMS && dbeta) atomicAdd(dbeta + c, sums[H + c]);
+  __syncthreads();
+  const bool vec = partial && !((uintptr_t)partial & 15);
+  for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
+    float4 a = *reinterpret_cast<const float4*>(sums + c);
+#pragma unroll 4
+    for (int t = 1; t < filled; ++t) {
+      const float4 b = *reinterpret_cast<const float4*>(sums + (size_t)t * width + c);
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    }
+    if (vec) {
+      *reinterpret_cast<float4*>(partial + (size_t)blockIdx.x * 2 * H + c) = a;
+      continue;
+    }
+    const float s[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {   // H is a multiple of 4: the four are all of d(gamma) or all of d(beta)
+      if (partial) partial[(size_t)blockIdx.x * 2 * H + c + j] = s[j];
+      else if (c < H && dgamma) atomicAdd(dgamma + c + j, s[j]);
+      else if (c >= H && dbeta) atomicAdd(dbeta + c - H + j, s[j]);
     }
   }
 }
@@ -559,8 +563,9 @@ static int norm_bwd_ring_launch(const void* dy, const void* x, const void* gamma
                                 const void* dres, void* dx, float* dgamma, float* dbeta, float* partial, int rows, int H, int G,
                                 int* used, cudaStream_t st) {
   auto kern = norm_bwd_ring_kernel<T, VPL, NW, RMS>;
-  const size_t ring = (size_t)(dres ? 2 * 3 : 3 * 2) * NW * VPL * 512, sums = (size_t)2 * H * sizeof(float);
-  const size_t smem = ring > sums ? ring : sums;
+  const size_t smem = (size_t)(dres ? 2 * 3 : 3 * 2) * NW * VPL * 512;
+  // the column sums of the teams take the ring's place: NW / G teams of 2 * H floats, H <= G * VPL * 512 / sizeof(T)
+  static_assert(2 * sizeof(float) / sizeof(T) <= 6, "column sums must fit into the ring");
   static bool configured = false;
   if (!configured) {
     TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
