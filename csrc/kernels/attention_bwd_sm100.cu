@@ -555,12 +555,12 @@ TB_EXPORT int tb_flash_attn_bwd(const void* q, const void* k, const void* v, con
   const int n_blk = (S + 127) / 128;
   const long grid = (long)n_blk * B * H;
   if (D == 64) {
-    static bool cfg = false;
-    if (!cfg) { TB_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaBwdSmem<64>::ALLOC)); cfg = true; }
+    static std::atomic<uint64_t> opted_in{0};
+    if (int e = smem_opt_in(opted_in, fa_bwd_kernel<64>, FaBwdSmem<64>::ALLOC)) return e;
     fa_bwd_kernel<64><<<(unsigned)grid, FB_THREADS, FaBwdSmem<64>::ALLOC, st>>>(mq, mk, mv, mdo, p);
   } else {
-    static bool cfg = false;
-    if (!cfg) { TB_CUDA_CHECK(cudaFuncSetAttribute(fa_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaBwdSmem<128>::ALLOC)); cfg = true; }
+    static std::atomic<uint64_t> opted_in{0};
+    if (int e = smem_opt_in(opted_in, fa_bwd_kernel<128>, FaBwdSmem<128>::ALLOC)) return e;
     fa_bwd_kernel<128><<<(unsigned)grid, FB_THREADS, FaBwdSmem<128>::ALLOC, st>>>(mq, mk, mv, mdo, p);
   }
   const long items = (long)B * S * H * (D / 8);

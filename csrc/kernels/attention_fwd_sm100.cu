@@ -686,11 +686,8 @@ TB_EXPORT int tb_flash_attn_fwd(const void* q, const void* k, const void* v, voi
   // 128-key blocks, D = 64: 7.7 us against 8.8).
 #define TB_FA(KERN, SMEM, THREADS, PER_SM)                                                                       \
   {                                                                                                              \
-    static bool cfg = false;                                                                                     \
-    if (!cfg) {                                                                                                  \
-      TB_CUDA_CHECK(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));              \
-      cfg = true;                                                                                                \
-    }                                                                                                            \
+    static std::atomic<uint64_t> opted_in{0};                                                                    \
+    if (int e = smem_opt_in(opted_in, KERN, SMEM)) return e;                                                     \
     const long slots = (long)(PER_SM)*sm_count();  /* persistent CTAs */                                         \
     KERN<<<(unsigned)(tiles < slots ? tiles : slots), THREADS, SMEM, st>>>(mq, mk, mv, p);                       \
   }

@@ -265,14 +265,11 @@ TB_EXPORT int tb_fsdp_unit_gather(const void* const* shards, void* unit_buf, con
   if (ctas > 128) ctas = 128;
   if (int r = tb_fill_gather(g, shards, unit_buf, flag_bufs, epoch_ptr, ready, chunk_bytes, cpr, 0, rank, world, ctas, status))
     return r;
-  static bool configured = false;
   constexpr int SMEM = GATHER_SMEM + 12 * 8 + 16 + 128;
-  if (!configured) {
-    TB_CUDA_CHECK(cudaFuncSetAttribute(fsdp_unit_gather_kernel<16384>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    TB_CUDA_CHECK(cudaFuncSetAttribute(fsdp_unit_gather_kernel<32768>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    TB_CUDA_CHECK(cudaFuncSetAttribute(fsdp_unit_gather_kernel<65536>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    configured = true;
-  }
+  static std::atomic<uint64_t> in16{0}, in32{0}, in64{0};
+  if (int r = smem_opt_in(in16, fsdp_unit_gather_kernel<16384>, SMEM)) return r;
+  if (int r = smem_opt_in(in32, fsdp_unit_gather_kernel<32768>, SMEM)) return r;
+  if (int r = smem_opt_in(in64, fsdp_unit_gather_kernel<65536>, SMEM)) return r;
   // piece size of the copy ring (experiment knob: TB_GATHER_PIECE_KB = 16, 32 or 64)
   static const int piece_kb = [] { const char* e = getenv("TB_GATHER_PIECE_KB"); return e ? atoi(e) : 16; }();
   if (piece_kb == 64 && chunk_bytes % 65536 == 0) fsdp_unit_gather_kernel<65536><<<ctas, 32, SMEM, st>>>(g);

@@ -484,11 +484,8 @@ gemm_pair_kernel(const __grid_constant__ Maps maps, const Params p) {
 template <int A_MAJOR, int B_MAJOR, bool COLSUM = false>
 static int launch(const Maps& maps, const Params& p, cudaStream_t stream) {
   auto kern = gemm_pair_kernel<A_MAJOR, B_MAJOR, COLSUM>;
-  static bool configured = false;
-  if (!configured) {
-    TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ALLOC));
-    configured = true;
-  }
+  static std::atomic<uint64_t> opted_in{0};
+  if (int r = smem_opt_in(opted_in, kern, ALLOC)) return r;
   const long total = (long)p.tiles_m * p.tiles_n * p.split_k;
   const int pairs = sm_count() / 2;
   kern<<<2 * (int)(total < pairs ? total : pairs), THREADS + (COLSUM ? 128 : 0), ALLOC, stream>>>(maps, p);

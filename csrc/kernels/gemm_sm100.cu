@@ -944,11 +944,8 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const OutMa
                        cudaStream_t stream) {
   using L = SmemLayout<BN, STAGES, GBUFS>;
   auto kern = gemm_bf16_kernel<BN, A_MAJOR, B_MAJOR, STAGES, GBUFS>;
-  static bool configured = false;
-  if (!configured) {
-    TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::ALLOC));
-    configured = true;
-  }
+  static std::atomic<uint64_t> opted_in{0};
+  if (int r = smem_opt_in(opted_in, kern, L::ALLOC)) return r;
   long total = (long)p.tiles_m * p.tiles_n * (p.stream_k ? p.kb_total : p.split_k);
   int workers = sm_count() - p.ag_ctas;  // copy CTAs and GEMM CTAs must all be resident at once
   if (workers < 1) TB_FAIL(TB_E_ARG, "gemm: too many copy CTAs");

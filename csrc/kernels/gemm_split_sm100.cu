@@ -253,11 +253,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 template <int A_MAJOR, int B_MAJOR>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t stream) {
   auto kern = gemm_split_kernel<A_MAJOR, B_MAJOR>;
-  static bool configured = false;
-  if (!configured) {
-    TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ALLOC));
-    configured = true;
-  }
+  static std::atomic<uint64_t> opted_in{0};
+  if (int r = smem_opt_in(opted_in, kern, ALLOC)) return r;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(p.tiles_m * p.tiles_n * p.S));
   cfg.blockDim = dim3(THREADS);

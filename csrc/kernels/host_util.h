@@ -76,6 +76,21 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// Opts a kernel in to `bytes` of dynamic shared memory, once per device: the attribute belongs to the kernel on one device,
+// so a process that works on a second one has to set it there, too. `done` is the kernel's own set of devices; a call costs
+// one cudaGetDevice.
+template <typename Kernel>
+inline int smem_opt_in(std::atomic<uint64_t>& done, Kernel* kern, int bytes) {
+  int dev = 0;
+  TB_CUDA_CHECK(cudaGetDevice(&dev));
+  const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;   // beyond 64 devices: set on every call
+  if (!(done.load(std::memory_order_acquire) & bit)) {
+    TB_CUDA_CHECK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.fetch_or(bit, std::memory_order_release);
+  }
+  return 0;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

@@ -566,11 +566,8 @@ static int norm_bwd_ring_launch(const void* dy, const void* x, const void* gamma
   const size_t smem = (size_t)(dres ? 2 * 3 : 3 * 2) * NW * VPL * 512;
   // the column sums of the teams take the ring's place: NW / G teams of 2 * H floats, H <= G * VPL * 512 / sizeof(T)
   static_assert(2 * sizeof(float) / sizeof(T) <= 6, "column sums must fit into the ring");
-  static bool configured = false;
-  if (!configured) {
-    TB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    configured = true;
-  }
+  static std::atomic<uint64_t> opted_in{0};
+  if (int r = smem_opt_in(opted_in, kern, 200 * 1024)) return r;
   const int teams = NW / G, want = (rows + teams - 1) / teams, cap = sm_count();  // never above norm_bwd_grid(rows)
   *used = want < cap ? want : cap;
   kern<<<*used, NW * 32, smem, st>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)dres, (T*)dx, dgamma, dbeta,

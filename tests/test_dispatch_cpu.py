@@ -1,6 +1,13 @@
 """Rules that pick a kernel or refuse a call, without a GPU: the launching functions are replaced by recorders."""
+import os
+import shutil
+import subprocess
+
 import pytest
 import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
 
 
 @pytest.fixture
@@ -54,3 +61,23 @@ def test_column_sums_refuse_other_buffers(monkeypatch):
     assert calls == []
     ew.colsum_into(x, torch.zeros(8))
     assert calls == ["tb_colsum"]
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or not os.path.exists(CUDA_INCLUDE), reason="needs g++ and the CUDA headers")
+def test_shared_memory_opt_in_is_per_device(tmp_path):
+    """More than 48 KB of shared memory is an attribute of a kernel on ONE device: a launcher that sets it once per process
+    fails on the second GPU. The helper runs against a fake runtime, and no launcher keeps a flag of its own."""
+    exe = str(tmp_path / "smem_opt_in_check")
+    src = os.path.join(ROOT, "tests", "native", "smem_opt_in_check.cpp")
+    build = subprocess.run(["g++", "-std=c++17", "-O1", "-I", CUDA_INCLUDE, "-I", os.path.join(ROOT, "csrc", "kernels"), src, "-o", exe],
+                           capture_output=True, text=True, timeout=300)
+    assert build.returncode == 0, build.stderr[-2000:]
+    run = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0, run.stdout
+    assert run.stdout.split() == ["0:100", "1:100", "1:200", "63:200", "2:100!", "2:100", "64:100", "64:100"]
+    kernels = os.path.join(ROOT, "csrc", "kernels")
+    for name in sorted(os.listdir(kernels)):
+        with open(os.path.join(kernels, name)) as f:
+            text = f.read()
+        assert not ("MaxDynamicSharedMemorySize" in text and "static bool" in text and "configured" in text), name
+        assert "static bool cfg" not in text, name
