@@ -505,6 +505,8 @@ bool gemm_pair_ok(const GemmArgs& a) {
   } else if (a.flags & (EPI_ATOMIC | EPI_ACCUM)) {
     return false;
   }
+  // rows that overlap (a residual expanded over the rows: stride 0) are for the kernels that read with plain loads
+  if (a.ldd < a.N || ((a.flags & EPI_RESIDUAL) && a.ldr < a.N)) return false;
   if (a.bias && !al16(a.bias)) return false;
   const bool res = a.flags & EPI_RESIDUAL, dgelu = a.flags & EPI_MUL_DGELU, pre = a.flags & EPI_STORE_PREACT;
   if (res + dgelu + pre > 1) return false;   // one auxiliary matrix through the two staging slots of a warp

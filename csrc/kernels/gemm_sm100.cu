@@ -1047,6 +1047,16 @@ static int route(const GemmArgs& a, int& bn, int& S) {
   return best;
 }
 
+// The kernel that tb_gemm_bf16 with bn = 0 takes for these sizes with 16-byte aligned operands: 0 the one of this file, 1 CTA
+// pairs, 2 + 16 * width + 4096 * S the cluster split. Touches no GPU.
+TB_EXPORT int tb_gemm_route(int M, int N, int K, int a_major, int b_major, int lda, int ldb, int ldd, int ldr, int flags, int split_k) {
+  void* p = (void*)256;
+  GemmArgs a{p, p, p, M, N, K, a_major, b_major, lda, ldb, ldd, p, p, ldr, p, p, flags, split_k, nullptr};
+  int bn = 0, S = 1;
+  const int r = g_dynamic_tiles || split_k < 0 ? ROUTE_ONE : route(a, bn, S);
+  return r == ROUTE_SPLIT ? 2 + 16 * bn + 4096 * S : r;
+}
+
 TB_EXPORT int tb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int a_major,
                            int b_major, int lda, int ldb, int ldd, const void* bias,
                            const void* residual, int ldr, void* preact, const void* aux, int flags,

@@ -81,3 +81,25 @@ def test_shared_memory_opt_in_is_per_device(tmp_path):
             text = f.read()
         assert not ("MaxDynamicSharedMemorySize" in text and "static bool" in text and "configured" in text), name
         assert "static bool cfg" not in text, name
+
+
+def _route(M, N, K, majors=(0, 0), flags=0, split_k=1, ldd=None, ldr=None):
+    """(kernel, tile width, K splits) that a product of these sizes runs on; 148 SMs are assumed without a GPU."""
+    from torsh_b200 import _native as nv
+    am, bm = majors
+    r = nv.cuda().tb_gemm_route(M, N, K, am, bm, M if am else K, N if bm else K, N if ldd is None else ldd, N if ldr is None else ldr,
+                                flags, split_k)
+    return ("one", 0, 1) if r == 0 else ("pair", 256, 1) if r == 1 else ("split", r % 4096 // 16, r // 4096)
+
+
+BIAS, GELU, RESIDUAL, OUT_F32, ATOMIC, PREACT, DGELU = 1, 2, 4, 8, 16, 32, 64
+
+
+def test_rows_that_overlap_stay_off_the_pair_kernel():
+    """Its residual comes through a tensor map, which takes no row stride below the row's length (an expanded residual has 0)."""
+    shape = (8192, 1024, 4096)
+    assert _route(*shape, flags=BIAS | RESIDUAL)[0] == "pair" and _route(*shape, flags=RESIDUAL, ldr=1032)[0] == "pair"
+    for ldr in (0, 8, 1016):
+        assert _route(*shape, flags=RESIDUAL, ldr=ldr)[0] == "one"
+    assert _route(*shape, ldr=0)[0] == "pair"   # no residual: its stride says nothing
+    assert _route(*shape, flags=OUT_F32 | ATOMIC, ldd=0)[0] == "one" and _route(*shape, ldd=0)[0] != "pair"

@@ -168,6 +168,17 @@ def test_weight_gradient_carries_the_bias_gradient(tokens, m, n, accumulate):
         assert _rel_elem(gw, rw) < 1e-2 and _rel_elem(gb, rb) < 1e-2
 
 
+@pytest.mark.parametrize("M", [13, 512, 4096])
+def test_residual_expanded_over_the_rows(M):
+    """One row added to every row of the product without being written out: a residual of row stride 0. One bf16 rounding."""
+    from torsh_b200.ops.linear import linear
+    torch.manual_seed(20)
+    x, w = torch.randn(2, M // 2 or 1, 1024, device=DEV, dtype=torch.bfloat16), torch.randn(4096, 1024, device=DEV, dtype=torch.bfloat16) / 32
+    row = torch.randn(4096, device=DEV, dtype=torch.bfloat16)
+    y = linear(x, w, residual=row.expand(*x.shape[:-1], 4096))
+    assert _rel_elem(y, x.float() @ w.float().t() + row.float()) < 1e-2
+
+
 @pytest.mark.parametrize("wmg,bmg", [((torch.bfloat16, (512, 256)), (torch.float32, (512,))), ((torch.float32, (256, 512)), (torch.float32, (512,))),
                                      ((torch.float32, (512, 256)), (torch.bfloat16, (512,))), ((torch.float32, (512, 256)), (torch.float32, (256,)))])
 def test_gradient_buffers_of_another_kind_are_refused(wmg, bmg):
