@@ -992,16 +992,26 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
                          const void* residual, int ldr, void* preact, const void* aux, int flags,
                          int split_k, int bn, int* status, cudaStream_t stream, const TpFusion& tp);
 
+// Tile width of the one-CTA kernel when the caller does not name one: 256-wide tiles halve the shared-memory traffic per
+// FLOP, 128 where they would leave SMs idle, 64 for outputs of at most 64 columns (64-channel convolutions: nothing is loaded or
+// multiplied for columns that do not exist).
+static int one_cta_bn(int M, int N, int split_k, bool narrow_ok) {
+  const long t256 = (long)((M + BM - 1) / BM) * ((N + 255) / 256) * split_k;
+  if (N <= 64 && narrow_ok) return 64;
+  return N > 128 && t256 >= sm_count() ? 256 : 128;
+}
+
 // Which kernel runs a plain product: the one of this file, CTA pairs on 256 x 256 tiles, or 128-row tiles with K split
-// over a cluster. The choice is the smallest of three modelled times (microseconds), fitted to measurements on an idle
-// B200 (fwd M x N x K: this kernel at its better width / pair / best split; cuBLAS is not involved):
+// over a cluster. The choice is the smallest of three modelled times (microseconds): a launch, and per wave of tiles the
+// larger of its K blocks and its epilogue. The constants were fitted to the three kernels' own times over 1981 products (M 1 to
+// 50 176, N 64 to 50 304, K 8 to 11 008, forward, input- and weight-gradient majors, with and without bias and residual; B200,
+// operands in L2); over these the choice costs 2.4 % more than always knowing the best kernel, and seven are more than 5 % behind
+// the one-CTA kernel, the worst 14 % (8 x 6400 x 1600, 11.4 against 13.0). Some of them (one-CTA / pair / best split):
 //   8192 x 4096 x 1024   58.7 / 55.2 / -         2048 x 4096 x 1024   20.8 / 18.4 / 40
 //   8192 x 1024 x 4096   58.0 / 53.2 / -         2048 x 1024 x 4096   20.5 / 26.0 / 21
 //   dgrad 2048 x 4096 x 22016  363 / 255 / -     1024 x 1024 x 4096   19.8 / 24.9 / 15.9
 //   13 x 1024 x 4096     18.8 / 23.0 / 6.9       256 x 1024 x 1024     9.5 / 10.6 / 6.5
-//   4096 x 1024 x 200     9.1 / 8.3 / -          1280 x 5120 x 104    11.4 / 12.3 / -
-// A pair needs 0.30 us per 64-wide K block of a wave of 74 tiles and at least 2.9 us for a wave's epilogue; this kernel
-// 0.25 us per K block of a wave of 148 tiles of 128 x 128 and at least 1.9 us.
+//   384 x 22016 x 4096   62.0 / 72.7 / -         8192 x 256 x 64       6.0 / - / 6.9
 enum : int { ROUTE_ONE = 0, ROUTE_PAIR = 1, ROUTE_SPLIT = 2 };
 
 static int route(const GemmArgs& a, int& bn, int& S) {
@@ -1013,20 +1023,26 @@ static int route(const GemmArgs& a, int& bn, int& S) {
   if (a.split_k > 1) return pair ? ROUTE_PAIR : ROUTE_ONE;  // the caller has dealt K itself
   const long kb = (a.K + BK - 1) / BK, sms = sm_count();
   auto waves = [](long n, long per) { return (double)((n + per - 1) / per); };
-  const double mn = a.b_major ? 1.1 : 1.0;  // MN-major B costs the one-CTA MMAs about a tenth
-  const long t256 = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
-  const long m128 = (a.M + 127) / 128, t128 = m128 * ((a.N + 127) / 128);
+  const double mn = a.b_major ? 1.04 : 1.0;  // MN-major operands cost 128-row MMAs a little
+  const double mn1 = a.a_major ? 1.05 * mn : mn;
+  // a second matrix in the epilogue goes through plain loads and stores there and through TMA on pairs
+  const double aux = a.flags & (EPI_RESIDUAL | EPI_MUL_DGELU | EPI_STORE_PREACT) ? 0.6 : 0.0;
+  const long m128 = (a.M + 127) / 128;
+  const int w1 = one_cta_bn(a.M, a.N, 1, true);
   int best = ROUTE_ONE;
-  double t = 5.0 + waves(t128, sms) * fmax(kb * (a.N <= 64 ? 0.18 : 0.25) * mn, 1.9);
-  if (pair) {
-    const double tp = 5.3 + waves(t256, sms / 2) * fmax(kb * 0.30 + 0.6, 2.9);
+  double t = 4.9 + waves(m128 * ((a.N + w1 - 1) / w1), sms) *
+                       (w1 == 256 ? fmax(kb * 0.39 * mn1, 5.4 + 2 * aux) : fmax(kb * (w1 == 64 ? 0.195 : 0.28) * mn1, 1.9 + aux));
+  if (pair && a.M > 128) {   // with fewer rows the second CTA of every pair has none
+    const long t256 = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
+    const double tp = 5.4 + waves(t256, sms / 2) * fmax(kb * 0.29 + 0.78, 3.1);
     if (tp < t) {
       t = tp;
       best = ROUTE_PAIR;
     }
   }
-  // A split CTA needs 0.18 (64 wide) or 0.25 us per K block, 0.6 us for the exchange and 3.5 us for every further wave, whose
-  // prologue nothing hides. Clusters of 4 and 8 do not fill every GPC: 120 and 112 CTAs at a time were seen on 148 SMs.
+  // A split CTA needs 0.17 (64 wide) or 0.29 us per K block, 0.6 us for the exchange or, without one, 1.7 us for writing 128 columns
+  // a thread, and 4.4 us for every further wave, whose prologue nothing hides. Clusters of 4 and 8 do not fill every GPC: 120 and
+  // 112 CTAs at a time were seen on 148 SMs.
   if (sms >= 128 && gemm_split_ok(a)) {
     for (int w = 64; w <= 128; w *= 2) {
       const long tiles = m128 * ((a.N + w - 1) / w);
@@ -1034,7 +1050,8 @@ static int route(const GemmArgs& a, int& bn, int& S) {
         const long cap = s <= 2 ? sms : s == 4 ? sms * 120 / 148 : sms * 112 / 148;
         const double wv = waves(tiles * s, cap);
         if (wv > 2) break;
-        const double ts = 5.2 + (s > 1 ? 0.6 : 0.0) + (wv - 1) * 3.5 + wv * (double)((kb + s - 1) / s) * (w == 64 ? 0.18 : 0.25) * mn;
+        const double ts = 5.7 + (s > 1 ? 0.6 : w == 128 ? 1.85 : 0.15) + (wv - 1) * 4.4 +
+                          wv * (double)((kb + s - 1) / s) * (w == 64 ? 0.17 : 0.29) * mn;
         if (ts < t) {
           t = ts;
           best = ROUTE_SPLIT;
@@ -1161,14 +1178,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   if (split_k < 1) split_k = 1;
   if (split_k > 1 && !(flags & EPI_ATOMIC)) TB_FAIL(TB_E_ARG, "tb_gemm_bf16: split_k > 1 needs EPI_ATOMIC");
   if (bn == 0 && stream_k) bn = N > 128 ? 256 : 128;
-  if (bn == 0) {
-    // 256-wide tiles halve the smem traffic per FLOP; fall back to 128 when that
-    // leaves SMs idle.
-    long t256 = (long)((M + BM - 1) / BM) * ((N + 255) / 256) * split_k;
-    bn = (N > 128 && t256 >= sm_count()) ? 256 : 128;
-    // narrow outputs (64-channel convolutions): nothing is loaded or multiplied for columns that do not exist
-    if (N <= 64 && (tp.kind == 0 || tp.kind == 3)) bn = 64;
-  }
+  if (bn == 0) bn = one_cta_bn(M, N, split_k, tp.kind == 0 || tp.kind == 3);
   if (bn != 64 && bn != 128 && bn != 256) TB_FAIL(TB_E_ARG, "tb_gemm_bf16: bn must be 128 or 256");
 
   GemmParams p{};

@@ -103,3 +103,17 @@ def test_rows_that_overlap_stay_off_the_pair_kernel():
         assert _route(*shape, flags=RESIDUAL, ldr=ldr)[0] == "one"
     assert _route(*shape, ldr=0)[0] == "pair"   # no residual: its stride says nothing
     assert _route(*shape, flags=OUT_F32 | ATOMIC, ldd=0)[0] == "one" and _route(*shape, ldd=0)[0] != "pair"
+
+
+@pytest.mark.parametrize("shape,kernel", [
+    ((8192, 4096, 1024), "pair"), ((8192, 1024, 4096), "pair"), ((2048, 4096, 1024), "pair"), ((4096, 50304, 1024), "pair"),
+    ((13, 1024, 4096), "split"), ((256, 1024, 1024), "split"), ((1024, 1024, 4096), "split"), ((64, 768, 3072), "split"),
+    # three rows of 128: 256-wide one-CTA tiles waste nothing (62 us, pairs 73)
+    ((384, 22016, 4096), "one"), ((384, 50304, 1024), "one"),
+    # one or two K blocks: what a CTA writes costs more than what it reads (6.0 us, one split CTA per tile 6.9)
+    ((8192, 256, 64), "one"), ((3136, 512, 128), "one"), ((1500, 1024, 256), "one"), ((512, 4096, 8), "one"),
+    # fewer rows than half a pair's
+    ((1, 50304, 768), "one"), ((128, 50304, 1024), "one")])
+def test_route_takes_the_faster_kernel(shape, kernel):
+    """Products timed on all three kernels, on both sides of where the choice changes."""
+    assert _route(*shape)[0] == kernel
