@@ -1018,6 +1018,27 @@ def test_gemm_measured_tile_selection():
         G.gemm_autotune(False)
 
 
+@pytest.mark.parametrize("shape", [(13, 1024, 4096), (2048, 4096, 1024)])
+def test_gemm_measured_selection_includes_the_launchers_choice(shape, monkeypatch):
+    """A table with tile records only (as an older run saved them) is completed with the kernel record, and the launcher's own
+    choice (a cluster split, CTA pairs) wins where it is the faster one; a hit measures nothing. The timer is a fake that makes
+    the launcher's choice the fastest."""
+    from torsh_b200.core.backend import Autotuner, TuneRecord
+    from torsh_b200.ops import gemm as G
+    M, N, K = shape
+    torch.manual_seed(5)
+    a, b = torch.randn(M, K, device=DEV, dtype=torch.bfloat16), torch.randn(N, K, device=DEV, dtype=torch.bfloat16)
+    ref, key = G.gemm(a, b), f"{M}x{N}x{K}|a0b0|f0"
+    ticks = iter([1.0, 2.0, 3.0])
+    tuner = Autotuner(timer=lambda fn: (fn(), next(ticks))[1])
+    tuner.table[f"gemm|{key}"] = TuneRecord(f"gemm|{key}", "bn128_r1", {"bn128_r0": 2.0, "bn128_r1": 1.0, "bn256_r0": 3.0, "bn256_r1": 4.0})
+    monkeypatch.setattr(G, "_autotune", tuner)
+    for _ in range(2):
+        assert torch.equal(G.gemm(a, b), ref)
+    rec = tuner.table[f"gemm-kernel|{key}"]
+    assert rec.choice == "bn0_r0" and set(rec.times_ms) == {"bn0_r0", "bn0_r1", "bn128_r1"} and len(tuner.table) == 2
+
+
 def test_jit_compiler_runs_fused_regions_as_generated_kernels(tmp_path_factory, monkeypatch):
     from torsh_b200 import jit_compiler as J
     monkeypatch.setenv("TORSH_JIT_DIR", str(tmp_path_factory.getbasetemp() / "jit"))

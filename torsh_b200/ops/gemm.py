@@ -29,10 +29,12 @@ EPI_RASTER_M = 256
 _configured = False
 
 # ---- measured tile selection --------------------------------------------------------------------------------------
-# Off by default: the launcher's heuristic (BN 256 unless the grid would be short, rasterise along M for wide outputs)
-# is what the benchmarks run. `gemm_autotune(True)` or TORSH_GEMM_AUTOTUNE=1 times the candidates (BN 128 / 256 x both
-# raster orders) once per problem shape on the caller's tensors and remembers the winner; TORSH_GEMM_TUNE_FILE keeps
-# the table across runs. Accumulating / atomic products and launches inside a CUDA-graph capture are never timed.
+# Off by default: the launcher chooses the kernel (one CTA per tile, CTA pairs, K split over a cluster) and its tile by modelled
+# times, and that is what the benchmarks run. `gemm_autotune(True)` or TORSH_GEMM_AUTOTUNE=1 times, once per problem shape and on
+# the caller's tensors, the one-CTA tiles (BN 128 / 256 x both raster orders), then the best of them against the launcher's own
+# choice in both orders, and remembers the winners; TORSH_GEMM_TUNE_FILE keeps the table across runs (a table without the second
+# kind of record is completed as its shapes come by). Accumulating / atomic products and launches inside a CUDA-graph capture are
+# never timed.
 _autotune = None
 
 
@@ -118,17 +120,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
     tuner = _env_autotune()
     if (tuner is not None and bn == 0 and raster_m is None and not atomic and not accumulate and split_k == 1
             and getattr(b, "_tb_fsdp_unit", None) is None and not torch.cuda.is_current_stream_capturing()):
-        key = f"gemm|{M}x{N}x{K}|a{a_major}b{b_major}|f{flags}"
-        rec = tuner.table.get(key)
+        shape = f"{M}x{N}x{K}|a{a_major}b{b_major}|f{flags}"
+        rec = tuner.table.get(f"gemm-kernel|{shape}")
         if rec is None:
             kw = dict(a_major=a_major, b_major=b_major, out=out, bias=bias, gelu=gelu, residual=residual, preact_out=preact_out,
                       dgelu_aux=dgelu_aux)
             cands = {f"bn{tbn}_r{int(r)}": (lambda tbn=tbn, r=r: gemm(a, b, bn=tbn, raster_m=r, **kw))
-                     for tbn in (128, 256) for r in (False, True)}
-            choice = tuner.select(key, cands)
+                     for tbn in (0, 128, 256) for r in (False, True)}
+            tile = tuner.select(f"gemm|{shape}", {k: f for k, f in cands.items() if not k.startswith("bn0")})
+            choice = tuner.select(f"gemm-kernel|{shape}", {k: cands[k] for k in ("bn0_r0", "bn0_r1", tile)})
         else:
             choice = rec.choice
-        bn, raster_m = int(choice[2:5]), choice.endswith("_r1")
+        bn, raster_m = int(choice[2:-3]), choice.endswith("_r1")
     if raster_m is None:
         raster_m = N > 4 * M or (N >= 16384 and N > M)
     if raster_m:
