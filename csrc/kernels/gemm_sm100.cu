@@ -1438,7 +1438,6 @@ TB_EXPORT int tb_ag_gemm(void* a_full, const void* const* shards, const void* co
   return 0;
 }
 
-// After a kernel gave up on a wait (status word set) its scheduler counters may not have been reset: clear them all.
 // Turns the dynamic tile scheduler of the persistent GEMM on (1) or off (0); returns the previous setting.
 TB_EXPORT int tb_gemm_set_dynamic(int on) {
   const int was = g_dynamic_tiles ? 1 : 0;
@@ -1446,6 +1445,9 @@ TB_EXPORT int tb_gemm_set_dynamic(int on) {
   return was;
 }
 
+TB_EXPORT int tb_gemm_dynamic() { return g_dynamic_tiles ? 1 : 0; }
+
+// After a kernel gave up on a wait (status word set) its scheduler counters may not have been reset: clear them all.
 TB_EXPORT int tb_gemm_reset_scheduler(cudaStream_t stream) {
   TB_ENSURE_DEVICE();
   unsigned* p = nullptr;

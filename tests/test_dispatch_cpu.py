@@ -18,6 +18,7 @@ def wgrad_calls(monkeypatch):
     monkeypatch.setattr(L, "gemm_wgrad_bias", lambda *a, **k: calls.append("wgrad_bias"))
     monkeypatch.setattr(L, "gemm", lambda a, b, **k: calls.append("gemm") or k.get("out"))
     monkeypatch.setattr(L.ew, "colsum_into", lambda *a: calls.append("colsum"))
+    monkeypatch.setattr(L, "dynamic_tiles", lambda: False)
     return calls
 
 
@@ -42,6 +43,25 @@ def test_bias_gradient_rides_only_into_fp32_buffers_of_the_right_shape(wgrad_cal
     dy, x, w, b = _layer(wmg, bmg)
     assert _wgrad_bgrad(dy, x, w, "nk", b, True, True) == (None, None)
     assert wgrad_calls == (["wgrad_bias"] if carried else ["gemm", "colsum"])
+
+
+@pytest.mark.parametrize("main_grads", [True, False])
+def test_dynamic_tiles_keep_weight_gradients_off_static_pairs(wgrad_calls, monkeypatch, main_grads):
+    """The switch asks for tiles that late CTAs can leave to others; pairs are dealt statically and hold two SMs each."""
+    from torsh_b200.ops import linear as L
+    m, n, tokens = 4096, 2304, 8192
+    w, b = torch.zeros(m, n, dtype=torch.bfloat16), torch.zeros(m, dtype=torch.bfloat16)
+    if main_grads:
+        w.main_grad, b.main_grad = torch.zeros(m, n), torch.zeros(m)
+    dy, x = torch.zeros(tokens, m, dtype=torch.bfloat16), torch.zeros(tokens, n, dtype=torch.bfloat16)
+    plans = []
+    monkeypatch.setattr(L, "gemm", lambda a, b, **k: plans.append((k.get("bn"), k.get("split_k", 1))) or torch.zeros(m, n))
+    monkeypatch.setattr(L, "dynamic_tiles", lambda: True)
+    L._wgrad_bgrad(dy, x, w, "nk", b, True, True)
+    assert "wgrad_bias" not in wgrad_calls and plans == [L._wgrad_plan(m, n, tokens)]
+    monkeypatch.setattr(L, "dynamic_tiles", lambda: False)
+    L._wgrad_bgrad(dy, x, w, "nk", b, True, True)
+    assert "wgrad_bias" in wgrad_calls
 
 
 def test_column_sums_refuse_other_buffers(monkeypatch):

@@ -56,6 +56,27 @@ def test_gemm_dynamic_tile_scheduler():
     assert _rel_elem(ref, a.float() @ b.float().t()) < 1e-2
 
 
+@pytest.mark.parametrize("main_grads", [False, True])
+def test_linear_gradients_with_dynamic_tiles(main_grads):
+    """Weight and bias gradients with the dynamic scheduler on: the one-CTA kernel and the column sums, the same values up to
+    one bf16 rounding (fresh gradients) or the order of fp32 sums (buffers that are added to)."""
+    from torsh_b200 import _native as nv
+    from torsh_b200.ops.linear import linear
+    torch.manual_seed(4)
+    x, dy = torch.randn(2048, 2304, device=DEV, dtype=torch.bfloat16), torch.randn(2048, 4096, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(4096, 2304, device=DEV) * 0.02).to(torch.bfloat16).requires_grad_(True)
+    b = torch.zeros(4096, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    if main_grads:
+        w.main_grad, b.main_grad = torch.zeros(4096, 2304, device=DEV), torch.zeros(4096, device=DEV)
+    was = nv.cuda().tb_gemm_set_dynamic(1)
+    try:
+        gw, gb = torch.autograd.grad(linear(x, w, b), (w, b), dy, allow_unused=True)
+    finally:
+        nv.cuda().tb_gemm_set_dynamic(was)
+    gw, gb, tol = (w.main_grad, b.main_grad, 1e-4) if main_grads else (gw, gb, 1e-2)
+    assert _rel_elem(gw, dy.float().t() @ x.float()) < tol and _rel_elem(gb, dy.float().sum(0)) < tol
+
+
 def test_gemm_epilogues():
     from torsh_b200.ops.gemm import gemm
     torch.manual_seed(2)

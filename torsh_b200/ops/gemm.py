@@ -160,6 +160,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_major: int = 0, b_major: int = 0
     return out
 
 
+def dynamic_tiles() -> bool:
+    """True while the persistent GEMM draws its tiles from a device counter (TB_GEMM_DYNAMIC, ``tb_gemm_set_dynamic``): for work
+    that shares the GPU with kernels of another stream. CTA pairs, whose tiles are dealt statically, are not used then."""
+    return bool(_lib().tb_gemm_dynamic())
+
+
 _WGRAD = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 6 + [ctypes.c_void_p] + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2
 
 

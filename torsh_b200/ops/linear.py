@@ -14,7 +14,7 @@ import torch
 
 from . import elementwise as ew
 from ._dispatch import kernel_ok
-from .gemm import gemm, gemm_wgrad_bias
+from .gemm import dynamic_tiles, gemm, gemm_wgrad_bias
 
 
 # TORSH_WGRAD_STREAM_K=0 goes back to uniform K-splits for the weight-gradient GEMMs
@@ -63,7 +63,7 @@ def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layout: st
     a, b = (dy2, x2) if layout == "nk" else (x2, dy2)
     m_out, n_out, k = a.shape[1], b.shape[1], a.shape[0]
     mg = getattr(weight, "main_grad", None)
-    if m_out >= 256 and n_out >= 256:
+    if m_out >= 256 and n_out >= 256 and not dynamic_tiles():
         bn, sk = 0, _wgrad_pair_split(m_out, n_out, k, mg is not None)
     else:
         bn, sk = _wgrad_plan(m_out, n_out, k)
@@ -101,7 +101,8 @@ def _wgrad_bgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor, layo
         m, n, k = dy2.shape[1], x2.shape[1], dy2.shape[0]
         wmg, bmg = getattr(weight, "main_grad", None), getattr(bias, "main_grad", None)
         tiles = ((m + 255) // 256) * ((n + 255) // 256)
-        if m >= 256 and n >= 256 and m % 8 == 0 and n % 8 == 0 and dy2.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0:
+        if (m >= 256 and n >= 256 and m % 8 == 0 and n % 8 == 0 and dy2.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0
+                and not dynamic_tiles()):
             if wmg is not None and bmg is not None:
                 if _adds_in_place(wmg, (m, n), dy2.device) and _adds_in_place(bmg, (m,), dy2.device):
                     gemm_wgrad_bias(dy2, x2, wmg, bmg, True, _wgrad_pair_split(m, n, k, True))
