@@ -312,20 +312,41 @@ __global__ void __launch_bounds__(THREADS) xent_ring_kernel(const T* logits, con
   }
 }
 
-// One CTA: valid = max(1, rows that are not ignored); loss = sum of the row losses * factor, or / valid when `mean`.
+// One cluster: valid = max(1, rows that are not ignored); loss = sum of the row losses * factor, or / valid when `mean`. The CTAs'
+// sums meet in rank order in the first CTA's registers, read through distributed shared memory.
 __global__ void __launch_bounds__(1024) xent_mean_kernel(const float* __restrict__ loss_rows, const long* __restrict__ targets,
                                                          int rows, long ignore_index, int mean, float factor,
                                                          float* __restrict__ loss, float* __restrict__ valid) {
   __shared__ float scratch[32];
+  __shared__ float2 part;
   float s = 0.f, n = 0.f;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < rows; i += 1024) {
+  for (long i = blockIdx.x * 1024 + threadIdx.x; i < rows; i += gridDim.x * 1024) {
     s += loss_rows[i];
     n += targets[i] != ignore_index ? 1.f : 0.f;
   }
   s = block_sum(s, scratch);
-  n = fmaxf(block_sum(n, scratch), 1.f);
-  if (threadIdx.x == 0) {
+  n = block_sum(n, scratch);
+  if (gridDim.x > 1) {   // the grid is one cluster
+    if (threadIdx.x == 0) part = make_float2(s, n);
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      s = n = 0.f;
+      for (unsigned r = 0; r < gridDim.x; ++r) {
+        float2 v;
+        asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %2, %3;\n ld.shared::cluster.v2.f32 {%0, %1}, [a];\n}"
+                     : "=f"(v.x), "=f"(v.y)
+                     : "r"((uint32_t)__cvta_generic_to_shared(&part)), "r"(r)
+                     : "memory");
+        s += v.x;
+        n += v.y;
+      }
+    }
+    // no CTA leaves while its sums may still be read
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    n = fmaxf(n, 1.f);
     *valid = n;
     *loss = mean ? s / n : s * factor;
   }
@@ -443,7 +464,24 @@ TB_EXPORT int tb_cross_entropy(const void* logits, const long* targets, float* l
 TB_EXPORT int tb_cross_entropy_mean(const float* loss_rows, const long* targets, int rows, long ignore_index, int mean,
                                     float factor, float* loss, float* valid, cudaStream_t st) {
   TB_ENSURE_DEVICE();
-  xent_mean_kernel<<<1, 1024, 0, st>>>(loss_rows, targets, rows < 0 ? 0 : rows, ignore_index, mean, factor, loss, valid);
+  // One SM takes in about 200 GB/s of the 12 bytes a row: eight as soon as that saves more than starting a cluster costs (one CTA
+  // and eight: 16 384 rows 3.2 and 3.8 us, 65 536 5.9 and 4.0, 1 000 000 58 and 12).
+  if (rows < 0) rows = 0;
+  if (rows < 32768) {
+    xent_mean_kernel<<<1, 1024, 0, st>>>(loss_rows, targets, rows, ignore_index, mean, factor, loss, valid);
+  } else {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(8);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 8;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, xent_mean_kernel, loss_rows, targets, rows, ignore_index, mean, factor, loss, valid));
+  }
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -527,6 +527,23 @@ def test_cross_entropy_in_place_reads_its_target_first(dtype, V):
     assert abs(loss.item() - ref.item()) < 1e-3
 
 
+@pytest.mark.parametrize("rows", [1023, 32767, 32768, 100003])
+def test_cross_entropy_mean_of_many_rows(rows):
+    """Both sides of the row count from which a cluster adds up the row losses, with and without ignored rows. The mean of
+    fp32 row losses (each within about 1e-6) in another order: 1e-5 of it."""
+    from torsh_b200.ops.softmax import cross_entropy
+    torch.manual_seed(26)
+    x = torch.randn(rows, 8, device=DEV)
+    tg = torch.randint(0, 8, (rows,), device=DEV)
+    full = torch.nn.functional.cross_entropy(x.double(), tg).item()
+    assert abs(cross_entropy(x, tg).item() - full) < 1e-5 * full
+    assert abs(cross_entropy(x, tg, root_scale=0.5).item() - 0.5 * full) < 1e-5 * full
+    tg[::3] = -100
+    some = torch.nn.functional.cross_entropy(x.double(), tg).item()
+    assert abs(cross_entropy(x, tg).item() - some) < 1e-5 * some
+    assert cross_entropy(x, torch.full_like(tg, -100)).item() == 0.0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("V", [40, 1000, 20011])
 def test_cross_entropy_masked_logits(dtype, V):
