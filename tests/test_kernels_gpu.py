@@ -544,6 +544,21 @@ def test_cross_entropy_mean_of_many_rows(rows):
     assert cross_entropy(x, torch.full_like(tg, -100)).item() == 0.0
 
 
+@pytest.mark.parametrize("inplace", [False, True])
+@pytest.mark.parametrize("V,width", [(1000, 1024), (60001, 60008)])
+def test_cross_entropy_of_columns_of_a_wider_buffer(V, width, inplace):
+    """Logits that are some of the columns of a buffer: the others keep their values, and the gradient is that of dense logits."""
+    from torsh_b200.ops.softmax import cross_entropy
+    torch.manual_seed(21)
+    wide = torch.randn(40, width + 16, device=DEV)
+    kept, tg = wide.clone(), torch.randint(0, V, (40,), device=DEV)
+    x = wide[:, 8:8 + V].requires_grad_(True)
+    (g,) = torch.autograd.grad(cross_entropy(x, tg, inplace_grad=inplace), x)
+    ref = kept[:, 8:8 + V].clone().requires_grad_(True)
+    torch.nn.functional.cross_entropy(ref, tg).backward()
+    assert g.shape == x.shape and _rel(g, ref.grad) < 1e-4 and torch.equal(wide, kept)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("V", [40, 1000, 20011])
 def test_cross_entropy_masked_logits(dtype, V):

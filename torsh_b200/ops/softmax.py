@@ -61,7 +61,13 @@ class _CrossEntropyFn(torch.autograd.Function):
         tg = targets.reshape(-1).contiguous().to(torch.int64)
         loss_rows = torch.empty(rows, dtype=torch.float32, device=logits.device)
         need_grad = logits.requires_grad
-        dl = (lg if inplace_grad else torch.empty_like(lg)) if need_grad else None
+        dl = None
+        if need_grad and lg.stride(0) > ld:
+            # rows of a wider buffer: the kernel fills every row of the gradient up to the stride, which must not be the
+            # neighbours' memory (in place) or lie beyond a dense buffer
+            dl = torch.empty(rows, lg.stride(0), dtype=lg.dtype, device=lg.device)[:, :ld]
+        elif need_grad:
+            dl = lg if inplace_grad else torch.empty_like(lg)
         # Generic path: the kernel writes the unscaled gradient and backward multiplies by
         # dloss / valid (both device scalars). With root_scale the caller promises that this loss
         # is the root of backward (upstream gradient 1) and that no target is ignored, so the
