@@ -358,6 +358,18 @@ def test_norm_bwd_teams(dtype, H, rows):
     assert _rel(gx, rx) < tol and _rel(gw, rw) < tol
 
 
+@pytest.mark.parametrize("which", ["weight", "bias"])
+@pytest.mark.parametrize("dtype,shape", [(torch.bfloat16, (512,)), (torch.float32, (256,))])
+def test_norm_gradient_buffers_of_another_kind_are_refused(which, dtype, shape):
+    from torsh_b200.ops.norm import layer_norm
+    x = torch.randn(8, 512, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    w, b = (torch.ones(512, device=DEV, dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+    w.main_grad, b.main_grad = torch.zeros(512, device=DEV), torch.zeros(512, device=DEV)
+    (w if which == "weight" else b).main_grad = torch.zeros(shape, device=DEV, dtype=dtype)
+    with pytest.raises(AssertionError):
+        torch.autograd.grad(layer_norm(x, w, b).sum(), (x, w, b), allow_unused=True)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("S", [129, 640, 1100])

@@ -73,6 +73,8 @@ def _norm_backward(ctx, dy, dres):
         return dx.view(ctx.shape), gw, gb, None, None
     # gradients of weight / bias accumulate straight into fp32 `main_grad` buffers when the
     # parameters carry them (flat mixed-precision storage); autograd then receives None
+    for mg in (wmg, bmg):   # the kernel adds fp32 values through the pointer
+        assert mg is None or (mg.dtype == torch.float32 and mg.numel() == H and mg.is_contiguous() and mg.device == x2.device)
     dgamma = wmg.view(-1) if wmg is not None else torch.zeros(H, dtype=torch.float32, device=x2.device)
     dbeta = None
     if ctx.has_bias:
