@@ -137,3 +137,34 @@ def test_rows_that_overlap_stay_off_the_pair_kernel():
 def test_route_takes_the_faster_kernel(shape, kernel):
     """Products timed on all three kernels, on both sides of where the choice changes."""
     assert _route(*shape)[0] == kernel
+
+
+def _params(test, name):
+    import test_kernels_gpu as G
+    marks = [m for m in getattr(G, test).pytestmark if m.name == "parametrize" and m.args[0] == name]
+    return marks[0].args[1]
+
+
+@pytest.mark.parametrize("test,kernel,flags", [
+    ("test_gemm_pair_tiles_and_epilogues", "pair", (0, BIAS | RESIDUAL, BIAS | GELU | PREACT, DGELU)),
+    ("test_gemm_cluster_split_k", "split", (0, BIAS | GELU | RESIDUAL | PREACT, DGELU)),
+    ("test_gemm_cluster_split_widths", "split", (0, BIAS | RESIDUAL)),
+    ("test_gemm_narrow_outputs", "one", (0, BIAS | RESIDUAL))])
+def test_gpu_tests_reach_the_kernel_that_they_name(test, kernel, flags):
+    """The GEMM tests choose their kernel by size: every product of theirs is on the kernel that it is there for."""
+    seen = set()
+    for shape in _params(test, "shape"):
+        for majors in _params(test, "majors"):
+            for f in flags:
+                r = _route(*shape, majors=majors, flags=f)
+                assert r[0] == kernel, (shape, majors, f, r)
+                seen.add(r[1:])
+    if test == "test_gemm_cluster_split_widths":
+        assert seen >= {(128, 4), (64, 2), (64, 8)}
+
+
+def test_wide_row_gemm_test_reaches_all_three_kernels():
+    shapes = _params("test_gemm_rows_wider_than_the_matrix", "shape")
+    for majors in _params("test_gemm_rows_wider_than_the_matrix", "majors"):
+        for f in (BIAS | RESIDUAL, BIAS | GELU | PREACT, DGELU):
+            assert [_route(*s, majors=majors, flags=f)[0] for s in shapes] == ["pair", "split", "one"]

@@ -296,6 +296,66 @@ def test_gemm_cluster_split_k(shape, majors):
     nv.check_status()
 
 
+@pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("shape", [(24, 3080, 1000), (200, 1000, 1024), (16, 2304, 768), (40, 72, 600), (72, 4104, 648)])
+def test_gemm_cluster_split_widths(shape, majors):
+    """Clusters of two, four and eight CTAs and both tile widths, every pairing of majors (test_dispatch_cpu.py holds that
+    these sizes run on the cluster kernel). One bf16 rounding, the same bits in every run."""
+    from torsh_b200.ops.gemm import gemm
+    torch.manual_seed(22)
+    M, N, K = shape
+    am, bm = majors
+    a = torch.randn((K, M) if am else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if bm else (N, K), device=DEV, dtype=torch.bfloat16) / K ** 0.5
+    bias, res = torch.randn(N, device=DEV, dtype=torch.bfloat16), torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    u = (a.float().t() if am else a.float()) @ (b.float() if bm else b.float().t())
+    out = gemm(a, b, a_major=am, b_major=bm, bias=bias, residual=res)
+    assert _rel_elem(out, u + bias.float() + res.float()) < 1e-2
+    assert torch.equal(out, gemm(a, b, a_major=am, b_major=bm, bias=bias, residual=res))
+    assert _rel_elem(gemm(a, b, a_major=am, b_major=bm), u) < 1e-2
+
+
+@pytest.mark.parametrize("majors", [(0, 0), (0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("shape", [(4104, 1032, 520), (200, 1000, 1024), (40000, 56, 72)])
+def test_gemm_rows_wider_than_the_matrix(shape, majors):
+    """Operands, output, pre-activation, residual and fp32 accumulator that are columns of wider buffers, on the pair, cluster
+    and one-CTA kernels: the strides are used and the columns beside them keep their values. One bf16 rounding; fp32 sums of
+    at most 1024 products differ by their order."""
+    from torsh_b200.ops.gemm import gemm
+    torch.manual_seed(23)
+    M, N, K = shape
+    am, bm = majors
+
+    def cols(r, c, extra, std=1.0, dtype=torch.bfloat16):
+        wide = (torch.randn(r, c + extra, device=DEV) * std).to(dtype)
+        return wide, wide[:, 8:8 + c]
+    _, a = cols(*((K, M) if am else (M, K)), 24)
+    _, b = cols(*((K, N) if bm else (N, K)), 40, K ** -0.5)
+    _, res = cols(M, N, 56)
+    bias, kw = torch.randn(N, device=DEV, dtype=torch.bfloat16), dict(a_major=am, b_major=bm)
+    u = (a.float().t() if am else a.float()) @ (b.float() if bm else b.float().t())
+
+    def check(wide, view, before, ref, tol):
+        assert _rel_elem(view, ref) < tol
+        assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + N:], before[:, 8 + N:])
+    wo, out = cols(M, N, 32)
+    wp, pre = cols(M, N, 32)
+    bo, bp = wo.clone(), wp.clone()
+    gemm(a, b, out=out, bias=bias, residual=res, **kw)
+    check(wo, out, bo, u + bias.float() + res.float(), 1e-2)
+    gemm(a, b, out=out, bias=bias, gelu=True, preact_out=pre, **kw)
+    check(wp, pre, bp, u + bias.float(), 1e-2)
+    check(wo, out, bo, torch.nn.functional.gelu(u + bias.float(), approximate="tanh"), 1e-2)
+    p = pre.float().requires_grad_(True)
+    torch.nn.functional.gelu(p, approximate="tanh").sum().backward()
+    gemm(a, b, out=out, dgelu_aux=pre, **kw)
+    check(wo, out, bo, u * p.grad, 1e-2)
+    wg, g = cols(M, N, 32, dtype=torch.float32)
+    bg = wg.clone()
+    gemm(a, b, out=g, atomic=True, **kw)
+    check(wg, g, bg, bg[:, 8:8 + N] + u, 1e-4)
+
+
 # ------------------------------------------------------------------ norms
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H", [256, 1024, 4096])
@@ -358,6 +418,27 @@ def test_norm_bwd_teams(dtype, H, rows):
     assert _rel(gx, rx) < tol and _rel(gw, rw) < tol
 
 
+@pytest.mark.parametrize("xd,wd,bd", [("bf16", "fp32", "fp32"), ("bf16", "fp32", "bf16"), ("bf16", "bf16", "fp32"), ("fp32", "bf16", "bf16"),
+                                      ("fp32", "bf16", "fp32")])
+@pytest.mark.parametrize("rows,H", [(3, 264), (700, 1024), (200, 5000)])
+def test_norm_gradients_in_the_parameters_dtype(xd, wd, bd, rows, H):
+    """Weights of another dtype than the rows: their gradients come out in their own dtype, written by the reduction when weight
+    and bias agree and cast from fp32 buffers when they do not. The weights are exact in bf16, so that only the rows, dx and
+    the gradients' own rounding (2^-9 in bf16) differ from the fp64 reference."""
+    from torsh_b200.ops.norm import layer_norm
+    torch.manual_seed(25)
+    t = dict(bf16=torch.bfloat16, fp32=torch.float32)
+    x = torch.randn(rows, H, device=DEV).to(t[xd]).requires_grad_(True)
+    w = (torch.randn(H, device=DEV) * 0.2 + 1).bfloat16().to(t[wd]).requires_grad_(True)
+    b = (torch.randn(H, device=DEV) * 0.1).bfloat16().to(t[bd]).requires_grad_(True)
+    dy = torch.randn(rows, H, device=DEV).to(t[xd])
+    grads = torch.autograd.grad(layer_norm(x, w, b, 1e-5), (x, w, b), dy)
+    r = [v.detach().double().requires_grad_(True) for v in (x, w, b)]
+    ref = torch.autograd.grad(torch.nn.functional.layer_norm(r[0], (H,), r[1], r[2], 1e-5), r, dy.double())
+    for g, v, want in zip(grads, (x, w, b), ref):
+        assert g.dtype == v.dtype and _rel(g, want) < (1e-2 if g.dtype == torch.bfloat16 else 1e-4)
+
+
 @pytest.mark.parametrize("which", ["weight", "bias"])
 @pytest.mark.parametrize("dtype,shape", [(torch.bfloat16, (512,)), (torch.float32, (256,))])
 def test_norm_gradient_buffers_of_another_kind_are_refused(which, dtype, shape):
@@ -394,6 +475,26 @@ def test_flash_attention_many_tiles(D, causal, S):
         assert _rel(out[b:b + 1], ref) < 2e-2
         for g, x in zip(grads, rg):
             assert ((g[b:b + 1].float() - x).norm() / x.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("B,S,H,D", [(3, 700, 16, 64), (2, 640, 20, 128), (20, 100, 12, 64), (2, 1100, 24, 128)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_flash_attention_packed_many_tiles(B, S, H, D, causal):
+    """The packed projection with more tiles than SMs (rows of 3 * H * D elements through the two-CTA forward), forward and
+    backward. P, O and the gradients carry bf16 roundings, as in the other attention tests."""
+    from torsh_b200.ops.attention import _sdpa_reference, flash_attention_qkvpacked
+    torch.manual_seed(24)
+    E = H * D
+    qkv = torch.randn(B * S, 3 * E, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    do = torch.randn(B * S, E, device=DEV, dtype=torch.bfloat16)
+    out = flash_attention_qkvpacked(qkv, B, S, H, D, causal=causal)
+    (g,) = torch.autograd.grad(out, qkv, do)
+    r = [qkv.detach()[:, i * E:(i + 1) * E].float().reshape(B, S, H, D).requires_grad_(True) for i in range(3)]
+    ref = _sdpa_reference(*r, causal, D ** -0.5)
+    assert _rel(out, ref.reshape(B * S, E)) < 2e-2
+    for i, x in enumerate(torch.autograd.grad(ref, r, do.float().reshape(B, S, H, D))):
+        x = x.reshape(B * S, E)
+        assert ((g[:, i * E:(i + 1) * E].float() - x).norm() / x.norm()).item() < 2e-2
 
 
 @pytest.mark.parametrize("B,S,H,D", [(2, 1, 3, 64), (3, 16, 5, 128), (2, 33, 2, 64), (1, 127, 3, 128), (2, 300, 4, 64), (2, 161, 3, 128)])
@@ -438,7 +539,7 @@ def test_rope_attention_packed_matches_separate_ops(B, S, H, D):
     (rg,) = torch.autograd.grad(ref, qkv, dy)
     assert torch.equal(out, ref)
     assert _rel(g, rg) < 1e-2
-    with torch.no_grad():   # a strided view is taken, too
+    with torch.no_grad():   # a strided view is accepted (and made dense first)
         wide = torch.cat([qkv, qkv], 1)
         assert torch.equal(rope_flash_attention_qkvpacked(wide[:, :3 * E], B, S, H, D, 10000.0), ref)
 
