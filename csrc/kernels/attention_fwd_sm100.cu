@@ -372,7 +372,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Two CTAs per SM, for launches of more tiles than SMs. A 128 x 128 block of scores costs 1024 clocks of exponentials and 512
+// Two CTAs per SM, for launches of enough tiles (fa_ctas_per_sm). A 128 x 128 block of scores costs 1024 clocks of exponentials and 512
 // (D = 64) or 1024 (D = 128) of MMA, and one CTA whose softmax warps all wait for the same score block at the same time took
 // about 3000 per block (latencies of the TMEM loads, the row-maximum exchange, the O read-back). Two CTAs of half the
 // size run out of step and fill each other's gaps, and the chain of one CTA is shorter:
@@ -667,6 +667,39 @@ using namespace tb;
 
 // q, k, v: bf16 views [B, S, H, D] with token strides q_stride / kv_stride (elements); head h starts
 // at element h*D of a token row; D in {64, 128}. o: [B*S, o_stride]. lse: fp32 [B, H, S] or null.
+// Which forward runs a launch: 1 or 2 CTAs per SM. One CTA with eight softmax warps finishes a tile sooner, two of half the size
+// use the SM better when both have work, so what decides is how the tiles come out: up to one per SM they are pure latency (72
+// tiles of three 128-key blocks, D = 64: 7.7 us against 8.8); with a causal mask and long sequences the longest tile alone decides
+// until there are about two per SM (D = 128, S 4096, 160 tiles 51 us with one CTA, 76 with two); an incomplete last round of at
+// most a tile per SM leaves every CTA alone (D = 128, S 3000 without a mask, 384 tiles 97 against 121). Both times are modelled as
+// the work of the CTA that is dealt the longest tiles, at measured costs (us): a launch, a tile and a 128-key block, for two
+// CTAs a block beside a busy one and alone. Over 722 launches of 149 to 1120 tiles and 1 to 32 blocks the choice costs 0.05 %
+// more than knowing the faster one; the worst, 1 block and 340 to 444 tiles with D = 64, 6 to 8 %. From 32 rounds on the last
+// one is below 2 % and two CTAs are taken.
+static int fa_ctas_per_sm(int B, int S, int H, int D, int causal) {
+  const long n_qb = (S + FA_BM - 1) / FA_BM, BH = (long)B * H, tiles = n_qb * BH, sms = sm_count();
+  if (tiles <= sms) return 1;
+  if (tiles > 32 * sms) return 2;
+  const bool wide = D == 128;
+  auto blocks = [&](long t) { return t >= tiles ? 0 : causal ? n_qb - t / BH : n_qb; };   // of tile t, long ones first
+  double one = wide ? 3.4 : 3.3;
+  for (long t = 0; t < tiles; t += sms) one += blocks(t) * (wide ? 1.16 : 1.075) + (wide ? 3.6 : 1.6);
+  const double beside = wide ? 2.36 : 1.78, alone = wide ? 2.03 : 1.20;
+  double two = 0;
+  for (long cta = 0; cta < 2 * sms; cta += 2 * sms - 1) {   // the first CTA and, where odd rounds are dealt backwards, the last
+    const long mate = cta < sms ? cta + sms : cta - sms;
+    double sum = wide ? 2.2 : 3.7;
+    for (long r = 0; r * 2 * sms < tiles; ++r) {
+      const bool back = wide && (r & 1);
+      const long n = blocks(r * 2 * sms + (back ? 2 * sms - 1 - cta : cta)), m = blocks(r * 2 * sms + (back ? 2 * sms - 1 - mate : mate));
+      if (n) sum += n * alone + (n < m ? n : m) * (beside - alone) + (wide ? 3.4 : 2.0) + (m ? (wide ? 1.95 : 0.3) : 0.0);
+    }
+    two = sum > two ? sum : two;
+  }
+  return one < two ? 1 : 2;
+}
+TB_EXPORT int tb_flash_attn_fwd_ctas(int B, int S, int H, int D, int causal) { return fa_ctas_per_sm(B, S, H, D, causal); }
+
 TB_EXPORT int tb_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B,
                                 int S, int H, int D, long q_stride, long kv_stride, long o_stride,
                                 float scale, int causal, int* status, cudaStream_t st) {
@@ -680,10 +713,7 @@ TB_EXPORT int tb_flash_attn_fwd(const void* q, const void* k, const void* v, voi
   if ((r = make_bshd_map(&mk, k, B, S, H, D, kv_stride))) return r;
   if ((r = make_bshd_map(&mv, v, B, S, H, D, kv_stride))) return r;
   FaFwdParams p{(__nv_bfloat16*)o, lse, B, S, H, o_stride, scale, causal, status};
-  const int n_qb = (S + FA_BM - 1) / FA_BM;
-  const long tiles = (long)n_qb * B * H;
-  // Tiles that do not even fill the SMs once are latency: eight softmax warps a tile finish it sooner (72 tiles of three
-  // 128-key blocks, D = 64: 7.7 us against 8.8).
+  const long tiles = (long)((S + FA_BM - 1) / FA_BM) * B * H;
 #define TB_FA(KERN, SMEM, THREADS, PER_SM)                                                                       \
   {                                                                                                              \
     static std::atomic<uint64_t> opted_in{0};                                                                    \
@@ -691,7 +721,7 @@ TB_EXPORT int tb_flash_attn_fwd(const void* q, const void* k, const void* v, voi
     const long slots = (long)(PER_SM)*sm_count();  /* persistent CTAs */                                         \
     KERN<<<(unsigned)(tiles < slots ? tiles : slots), THREADS, SMEM, st>>>(mq, mk, mv, p);                       \
   }
-  if (tiles <= sm_count()) {
+  if (fa_ctas_per_sm(B, S, H, D, causal) == 1) {
     if (D == 64) TB_FA(fa_fwd_kernel<64>, FaFwdSmem<64>::ALLOC, FA_THREADS, 1)
     else TB_FA(fa_fwd_kernel<128>, FaFwdSmem<128>::ALLOC, FA_THREADS, 1)
   } else {

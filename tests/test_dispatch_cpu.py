@@ -168,3 +168,26 @@ def test_wide_row_gemm_test_reaches_all_three_kernels():
     for majors in _params("test_gemm_rows_wider_than_the_matrix", "majors"):
         for f in (BIAS | RESIDUAL, BIAS | GELU | PREACT, DGELU):
             assert [_route(*s, majors=majors, flags=f)[0] for s in shapes] == ["pair", "split", "one"]
+
+
+@pytest.mark.parametrize("B,S,H,D,causal,ctas", [
+    (1, 384, 24, 64, 0, 1), (1, 1024, 18, 128, 1, 1),                              # at most a tile per SM
+    (1, 2048, 10, 128, 1, 1), (1, 4096, 9, 128, 1, 1), (1, 2048, 10, 64, 1, 1),    # the longest tile decides
+    (1, 4096, 12, 128, 0, 1), (1, 3000, 25, 128, 0, 1),                            # a last round that leaves CTAs alone
+    (1, 2048, 15, 64, 1, 2), (1, 700, 48, 128, 1, 2), (1, 256, 100, 128, 0, 2), (1, 4096, 18, 128, 0, 2),
+    (8, 1024, 16, 64, 1, 2), (3, 1531, 12, 64, 0, 2), (2, 4096, 16, 128, 1, 2), (1, 2048, 32, 128, 1, 2),
+    (16, 4096, 32, 128, 0, 2), (64, 128, 64, 64, 1, 2)])
+def test_attention_forward_takes_the_faster_kernel(B, S, H, D, causal, ctas):
+    """Launches timed on both forward kernels (one and two CTAs per SM), on both sides of where the choice changes."""
+    from torsh_b200 import _native as nv
+    assert nv.cuda().tb_flash_attn_fwd_ctas(B, S, H, D, causal) == ctas
+
+
+def test_attention_gpu_tests_reach_both_forward_kernels():
+    from torsh_b200 import _native as nv
+    ctas = nv.cuda().tb_flash_attn_fwd_ctas
+    many = {ctas(5, S, 32, D, c) for S in _params("test_flash_attention_many_tiles", "S") for D in (64, 128) for c in (0, 1)}
+    assert many == {2}
+    packed = [(B * H * -(-S // 128), ctas(B, S, H, D, c)) for B, S, H, D in _params("test_flash_attention_packed_many_tiles", "B,S,H,D")
+              for c in (0, 1)]
+    assert all(tiles > 148 for tiles, _ in packed) and {k for _, k in packed} == {1, 2}
