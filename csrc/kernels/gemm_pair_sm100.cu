@@ -3,7 +3,7 @@
 // Two CTAs of one cluster (the two SMs of a TPC) work on one 256 x 256 tile. Each loads its own 128 rows of A and its own
 // 128 rows of B, and the tensor cores of both SMs read both halves of B, so a K block costs each SM 32 KB of shared
 // memory traffic where the one-CTA 128 x 256 tile costs 48 KB: 1.5x the arithmetic per byte staged. That is what bounds
-// the one-CTA kernel at large sizes (measured on 8192 x 4096 x 1024, see gemm_dispatch in gemm_sm100.cu for both sides).
+// the one-CTA kernel at large sizes (measured on both sides at route() in gemm_sm100.cu).
 //
 // 320 threads per CTA, persistent over a static deal of the tiles:
 //   warp 0      TMA producer of this CTA's A and B halves; every copy reports to the full barrier of the pair's leader

@@ -587,7 +587,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
           for (int c = 0; c < BN / 64; ++c) {
             const int col = n_t * BN + c * 64, t9 = col / cin;
-            if (t9 >= 9) b_chunks = min(b_chunks, c);   // nothing is loaded past the last tap (those rows stay zero)
+            if (t9 >= 9) b_chunks = min(b_chunks, c);   // nothing is loaded past the last tap: those columns of D are not stored
             b_ci[c] = col - t9 * cin;
             b_kh[c] = t9 / 3 - 1;
             b_kw[c] = t9 - t9 / 3 * 3 - 1;

@@ -1,10 +1,10 @@
 // LayerNorm and RMSNorm forward / backward for sm_100a.
 //
-// One CTA walks rows (grid-stride); each thread owns up to VPT 16-byte vectors of the row and
-// keeps them in registers, so every element is read from HBM exactly once per pass. Row
-// statistics use two block reductions (mean, then centred variance) for accuracy. The backward
-// keeps per-thread fp32 partial sums of d(gamma) / d(beta) for its own columns across all rows of
-// the CTA and flushes them once with atomics into fp32 gradient buffers.
+// Every element is read from HBM exactly once per pass and the row statistics are a mean and then a centred variance, for
+// accuracy. Rows of up to 256 vectors of 16 bytes are a warp each in the forward, wider ones a CTA. The backward gives rows of up
+// to 8192 elements to teams of warps that copy them ahead through a ring in shared memory, wider ones to a CTA; both keep fp32
+// partial sums of d(gamma) / d(beta) in registers over all their rows and leave one partial row per CTA, which a second kernel
+// adds up (atomics only where the caller gives no workspace).
 //
 // Semantics follow the reference layers: LayerNorm eps 1e-5 (biased variance) and
 // RMSNorm y = x / sqrt(mean(x^2) + eps) * w with eps 1e-6

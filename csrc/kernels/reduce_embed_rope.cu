@@ -148,10 +148,6 @@ __global__ void gnn_scatter_kernel(const T* __restrict__ x, const long* __restri
   }
 }
 
-// Rotary embedding on x [B, S, heads, D] (in place allowed). Adjacent pairs (2i, 2i+1) rotate by
-// pos * base^(-2i/D): the pairing and frequency rule of RotaryPositionalEmbedding
-// (crates/torsh-nn/src/layers/embedding.rs:372-430), whose rotate step is a no-op in the
-// reference. sign = -1 applies the inverse rotation (the backward pass).
 // Rotation of the q and k bands of a packed projection output [tokens, 3 * heads * D] (q | k | v, head-major), the v band
 // copied (nbands = 3) or left alone (nbands = 2, in place: every element is read and written by the same thread). A thread
 // evaluates the angles of 8 neighbouring columns once and turns them for ROPE_HEADS heads: slicing the bands out, turning them
@@ -203,6 +199,10 @@ __global__ void rope_qkv_kernel(const bf16* x, bf16* y, long tokens, int S, int 
   }
 }
 
+// Rotary embedding on x [B, S, heads, D] (in place allowed). Adjacent pairs (2i, 2i+1) rotate by
+// pos * base^(-2i/D): the pairing and frequency rule of RotaryPositionalEmbedding
+// (crates/torsh-nn/src/layers/embedding.rs:372-430), whose rotate step is a no-op in the
+// reference. sign = -1 applies the inverse rotation (the backward pass).
 template <typename T>
 __global__ void rope_kernel(const T* __restrict__ x, T* __restrict__ y, long B, int S, int heads,
                             int D, float base, int pos_offset, float sign) {

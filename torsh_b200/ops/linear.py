@@ -17,13 +17,14 @@ from ._dispatch import kernel_ok
 from .gemm import dynamic_tiles, gemm, gemm_wgrad_bias
 
 
-# TORSH_WGRAD_STREAM_K=0 goes back to uniform K-splits for the weight-gradient GEMMs
+# TORSH_WGRAD_STREAM_K=0 goes back to uniform K-splits for the weight gradients of the one-CTA kernel
 _STREAM_K = os.environ.get("TORSH_WGRAD_STREAM_K", "1") != "0"
 
 
 def _wgrad_plan(m_out: int, n_out: int, k: int) -> tuple[int, int]:
-    """(tile width, split-K factor) for a weight-gradient GEMM: wide tiles when the output is wide
-    enough, and enough K-splits that the work units fill the 148 SMs about twice."""
+    """(tile width, split-K factor) for a weight-gradient GEMM on the one-CTA kernel: wide tiles when the output is wide enough,
+    and enough K-splits that the work units fill the 148 SMs about twice. Outputs that fill 256 x 256 tiles come here only
+    while tiles are dealt dynamically; otherwise they run on CTA pairs (:func:`_wgrad_pair_split`)."""
     bn = 256 if n_out >= 256 else 128
     tiles = ((m_out + 127) // 128) * ((n_out + bn - 1) // bn)
     kb = (k + 63) // 64
