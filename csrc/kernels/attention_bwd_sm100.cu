@@ -329,13 +329,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     for (int t = 0; t < n_it; ++t) {
       mbar_wait(dq_full, t & 1, abort_flag, p.status, TB_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
-      const int row0 = (i0 + t) * 128 + (warp & 3) * 32, rows = min(32, p.S - row0);
-      if (rows <= 0) {   // nothing of this warp's quarter is in the sequence
-        tc_fence_before();
-        mbar_arrive(dq_empty);
-        continue;
-      }
-      float* dq_grp = p.dQ_acc + ((size_t)bh * p.S + row0) * D;
 #pragma unroll
       for (int c = 0; c < D / 32; c += 2) {
         // both columns groups to registers first: with the last pair the columns are free before anything is staged
@@ -358,11 +351,17 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
+          // worked out here and not once per block: held across the block, the row count and the pointer cost the compute warps
+          // registers (D = 128: spills, 0.5 to 1.5 us of a launch)
+          const int row0 = (i0 + t) * 128 + (warp & 3) * 32, rows = min(32, p.S - row0);
+          float* dq_grp = p.dQ_acc + ((size_t)bh * p.S + row0) * D;
+          if (rows > 0) {   // else nothing of this warp's quarter is in the sequence
 #pragma unroll
-          for (int k = 0; k < 2; ++k)
-            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_grp + (c + k) * rows * 32),
-                         "r"(smem_u32(stage + k * 4096)), "r"(rows * 128)
-                         : "memory");
+            for (int k = 0; k < 2; ++k)
+              asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dq_grp + (c + k) * rows * 32),
+                           "r"(smem_u32(stage + k * 4096)), "r"(rows * 128)
+                           : "memory");
+          }
           bulk_commit();
         }
       }
