@@ -310,7 +310,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
 }
 
-template <typename T, int VPL, int NW, bool RMS>
+// ONE: a CTA of a single team, one row per CTA.
+template <typename T, int VPL, int NW, bool RMS, bool ONE>
 __global__ void __launch_bounds__(NW * 32, 1) norm_bwd_ring_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma, const float* __restrict__ mean_in,
     const float* __restrict__ rstd_in, const T* __restrict__ dres, T* __restrict__ dx, float* __restrict__ dgamma,
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(NW * 32, 1) norm_bwd_ring_kernel(
   extern __shared__ __align__(16) uint8_t nb_smem[];
   __shared__ float2 exch[2][NW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int teams = NW / G, team = warp / G, member = warp - team * G;
+  const int teams = ONE ? 1 : NW / G, team = ONE ? 0 : warp / G, member = warp - team * G;
   const int nvec = H / N, narr = dres ? 3 : 2, stages = dres ? 2 : 3;
   const bool active = team < teams;
   const int step = gridDim.x * teams;
@@ -562,16 +563,19 @@ template <typename T, int VPL, int NW, bool RMS>
 static int norm_bwd_ring_launch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
                                 const void* dres, void* dx, float* dgamma, float* dbeta, float* partial, int rows, int H, int G,
                                 int* used, cudaStream_t st) {
-  auto kern = norm_bwd_ring_kernel<T, VPL, NW, RMS>;
+  // No more rows than SMs: a CTA of one team each starts and ends sooner than a few of 16 or 24 warps (LayerNorm 16 x 1024 fp32
+  // with gradients that accumulate 8.8 -> 7.8 us, 100 x 1600 fp32 8.4 -> 7.6, 16 x 1600 bf16 9.6 -> 8.7).
+  const bool one = rows <= sm_count();
+  auto kern = one ? norm_bwd_ring_kernel<T, VPL, NW, RMS, true> : norm_bwd_ring_kernel<T, VPL, NW, RMS, false>;
   const size_t smem = (size_t)(dres ? 2 * 3 : 3 * 2) * NW * VPL * 512;
   // the column sums of the teams take the ring's place: NW / G teams of 2 * H floats, H <= G * VPL * 512 / sizeof(T)
   static_assert(2 * sizeof(float) / sizeof(T) <= 6, "column sums must fit into the ring");
-  static std::atomic<uint64_t> opted_in{0};
-  if (int r = smem_opt_in(opted_in, kern, 200 * 1024)) return r;
-  const int teams = NW / G, want = (rows + teams - 1) / teams, cap = sm_count();  // never above norm_bwd_grid(rows)
+  static std::atomic<uint64_t> in_one{0}, in_many{0};
+  if (int r = smem_opt_in(one ? in_one : in_many, kern, 200 * 1024)) return r;
+  const int teams = one ? 1 : NW / G, want = (rows + teams - 1) / teams, cap = sm_count();  // never above norm_bwd_grid(rows)
   *used = want < cap ? want : cap;
-  kern<<<*used, NW * 32, smem, st>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)dres, (T*)dx, dgamma, dbeta,
-                                    partial, rows, H, G);
+  kern<<<*used, (one ? G : NW) * 32, smem, st>>>((const T*)dy, (const T*)x, (const T*)gamma, mean, rstd, (const T*)dres, (T*)dx, dgamma,
+                                                 dbeta, partial, rows, H, G);
   TB_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -439,6 +439,27 @@ def test_norm_gradients_in_the_parameters_dtype(xd, wd, bd, rows, H):
         assert g.dtype == v.dtype and _rel(g, want) < (1e-2 if g.dtype == torch.bfloat16 else 1e-4)
 
 
+@pytest.mark.parametrize("rows,H", [(1, 264), (5, 1024), (700, 264), (2000, 4104)])
+@pytest.mark.parametrize("rms", [0, 1])
+def test_norm_bwd_workspace_forms(rows, H, rms):
+    """The launcher's workspace 16-byte aligned, off that alignment and absent (atomics), with one and with several teams a
+    CTA: the same gradients up to the order of fp32 sums of at most 2000 terms."""
+    from torsh_b200 import _native as nv
+    from torsh_b200.ops import norm as N
+    torch.manual_seed(27)
+    x, dy = (torch.randn(rows, H, device=DEV) for _ in range(2))
+    w, mean = torch.randn(H, device=DEV), x.mean(1) * (1 - rms)
+    rstd = torch.rsqrt((x - mean[:, None]).square().mean(1) + 1e-5)
+    ws = torch.empty(N._workspace_elems(rows, H) + 4, device=DEV)
+    xh = ((x - mean[:, None]) * rstd[:, None]).double()
+    want = ((dy.double() * xh).sum(0) + 1, dy.double().sum(0) + 1)
+    for workspace in (ws.data_ptr(), ws.data_ptr() + 4, None):
+        dx, dg, db = torch.empty_like(x), torch.ones(H, device=DEV), torch.ones(H, device=DEV)
+        N.call("tb_norm_bwd", N._BWD, dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(), None, dx.data_ptr(),
+               dg.data_ptr(), None if rms else db.data_ptr(), workspace, rows, H, rms, 1, nv.stream_ptr())
+        assert _rel(dg, want[0]) < 1e-5 and (rms or _rel(db, want[1]) < 1e-5)
+
+
 @pytest.mark.parametrize("which", ["weight", "bias"])
 @pytest.mark.parametrize("dtype,shape", [(torch.bfloat16, (512,)), (torch.float32, (256,))])
 def test_norm_gradient_buffers_of_another_kind_are_refused(which, dtype, shape):
